@@ -500,11 +500,11 @@ fz::StageArgs<R> stage_args(fz_handle* h, int stage) {
   a.zoff[0] = 0;
   for (int c = 0; c < h->zchunks && c < fz::FZ_MAX_ZCHUNKS; c++) a.zoff[c + 1] = a.zoff[c] + h->zsizes[(size_t)c];
   const fz_params& p = h->prm;
-  a.dt_h = (R)(p.dt / p.h);
-  a.frc2 = (R)(0.5 * p.rho * p.c * p.c);
-  a.firho = (R)(0.5 / p.rho);
-  a.fc = (R)(0.5 * p.c);
-  a.inv_h = (R)(1.0 / p.h);
+  a.z0 = (R)(p.rho * p.c);
+  a.dt_p = (R)(0.5 * p.dt * p.c / p.h);
+  a.dt_v = (R)(0.5 * p.dt / (p.h * p.rho));
+  a.ih_p = (R)(0.5 * p.c / p.h);
+  a.ih_v = (R)(0.5 / (p.h * p.rho));
   const double w = (stage == 0) ? 1.0 : (stage == 1) ? 0.25 : 2.0 / 3.0;
   a.wdt = (R)(w * p.dt);
   a.pml_on = h->pml_on ? 1 : 0;

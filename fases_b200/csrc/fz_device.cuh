@@ -86,11 +86,11 @@ struct StageArgs {
   // chunk c of a member covers its interior planes [zoff[c], zoff[c+1]) (counted from the first
   // interior plane); chunks may differ in length (long ones first, short ones for the last waves)
   int32_t zoff[FZ_MAX_ZCHUNKS + 1];
-  R dt_h;   // dt / h
-  R frc2;   // 0.5 * rho * c^2
-  R firho;  // 0.5 / rho
-  R fc;     // 0.5 * c
-  R inv_h;  // 1 / h
+  R z0;     // rho * c
+  R dt_p;   // dt / h * c / 2: p per difference of the characteristics
+  R dt_v;   // dt / h / (2 rho): velocity per sum of the characteristics
+  R ih_p;   // 1 / h * c / 2 (the cPML's flux differences)
+  R ih_v;   // 1 / h / (2 rho)
   R wdt;    // stage weight * dt (cPML correction weight)
   // cPML (pml_on = 0: no face enabled)
   int32_t pml_on;

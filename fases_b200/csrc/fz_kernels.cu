@@ -28,9 +28,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -86,16 +83,15 @@ __device__ __noinline__ void drain_ring(uint64_t* mbar, int it_fail, int nplanes
 // Shared-memory layout of the stage kernel.
 template <class R>
 struct StageSmem {
-  typedef typename Pair<R>::T P;
   // one field of one plane tile, padded to a multiple of 128 bytes (TMA destinations)
   static constexpr int FIELD = ((PH * PW * (int)sizeof(R) + 127) / 128) * 128;  // halo tile
   static constexpr int OWN = ((TX * TY * (int)sizeof(R) + 127) / 128) * 128;     // own tile
   static constexpr int CLSB = ((TX * TY + 127) / 128) * 128;                     // class bytes
   static constexpr int BUF = 3 * FIELD + 4 * OWN + CLSB;         // p,u,v halo | U0 own | cls
   static constexpr int TILES = NBUF * BUF;
-  static constexpr int XC = TY * (TX + 2) * (int)sizeof(P);        // one V array of x-centres
-  static constexpr int YC = (TY + 2) * TX * (int)sizeof(P);        // one V array of y-centres
-  static constexpr int CENTRES = 2 * (2 * XC + 2 * YC);            // double buffered (m, p) x and y
+  static constexpr int XC = TY * (TX + 2);                         // one characteristic of the x-centres
+  static constexpr int YC = (TY + 2) * TX;                         // one characteristic of the y-centres
+  static constexpr int CENTRES = 2 * (2 * XC + 2 * YC) * (int)sizeof(R);  // double buffered (wr, wl) x and y
   static constexpr int BYTES = TILES + CENTRES + 64 + 128;         // + mbarriers + base alignment
 };
 
@@ -221,29 +217,15 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
   // earlier; plane it_fail + 2 is issued only after the abort check) -- so that no copy lands in
   // shared memory after the block has gone. If that wait runs out as well, the block exits
   // anyway and the error word already says that the results are invalid.
-#if defined(FZ_V_SPLITBAR)
-  __shared__ __align__(8) uint64_t cbar[2];  // centre buffers: one arrival per warp
-  __shared__ int s_abort;
-#endif
   if (lt == 0) {
     for (int b = 0; b < NBUF; ++b) mbar_init(&mbar[b], 1);
-#if defined(FZ_V_SPLITBAR)
-    mbar_init(&cbar[0], NTHREADS / 32);
-    mbar_init(&cbar[1], NTHREADS / 32);
-#endif
     fence_mbar_init();
-#if defined(FZ_V_SPLITBAR)
-    s_abort = 0;
-#endif
   }
   __syncthreads();
   if (lt == 0) {
     issue(0);
     if (nplanes > 1) issue(1);
   }
-
-  const P kA = pmk(A.frc2, A.firho);
-  const P kC = psplat<R>(-A.fc);
 
   // z-queue loads: a column outside the grid (a ragged tile edge) reads the grid's last column
   // instead, so the loads need no test; such a thread stores nothing
@@ -254,18 +236,17 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
     return pmk(A.pi[g], A.wi[g]);
   };
 
-  // z prologue: centres kb-1 and kb give the flux through face kb-1/2 and V-(kb+1/2).
+  // z prologue: centres kb-1 and kb give the characteristics at face kb-1/2 and wr at kb+1/2.
   const P zero = psplat<R>(R(0));
-  P qa = zero, qb = zero, qc = zero, qd = zero, qe_next = zero, zm = zero, Fz_lo = zero;
+  P qa = zero, qb = zero, qc = zero, qd = zero, qe_next = zero;
+  R zr_lo = R(0), zr = R(0), zl = R(0);  // wr(k-1), wr(k), wl(k)
   if (!DIM2) {
     const P z0 = ld_pw(kb - 3), z1 = ld_pw(kb - 2), z2 = ld_pw(kb - 1), z3 = ld_pw(kb), z4 = ld_pw(kb + 1);
     const P z5 = ld_pw(kb + 2);
     qe_next = ld_pw(kb + 3);
-    P m0, p0, m1, p1;
-    weno_center<R>(z0, z1, z2, z3, z4, m0, p0);
-    weno_center<R>(z1, z2, z3, z4, z5, m1, p1);
-    Fz_lo = godunov<R>(m0, p1, kA, kC);
-    zm = m1;
+    R unused;
+    weno_waves<R, WENO_LO>(z0, z1, z2, z3, z4, A.z0, zr_lo, unused);
+    weno_waves<R>(z1, z2, z3, z4, z5, A.z0, zr, zl);
     // queue of plane values k-1 .. k+2 for the centre of plane k+1
     qa = z2; qb = z3; qc = z4; qd = z5;
   }
@@ -282,22 +263,18 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
   int64_t gz = colz + plane * (kb + 4);  // z-queue load of the next iteration (plane k + 4)
   for (int it = 0; it < nplanes; ++it, gk += plane, gz += plane) {
     const int k = kb + it;
-    P* XCm = reinterpret_cast<P*>(cbase + (it & 1) * (2 * L::XC + 2 * L::YC));
-    P* XCp = XCm + TY * (TX + 2);
-    P* YCm = XCp + TY * (TX + 2);
-    P* YCp = YCm + (TY + 2) * TX;
+    R* XR = reinterpret_cast<R*>(cbase) + (it & 1) * (2 * L::XC + 2 * L::YC);
+    R* XL = XR + L::XC;
+    R* YR = XL + L::XC;
+    R* YL = YR + L::YC;
 
     // ---- register loads for this plane (prefetched) and the next one
     const P qe = qe_next;
-    P vmC = zero, Fz_hi = zero;
+    R zr_hi = R(0), zl_hi = R(0);
     if (!DIM2) {
       if (it + 1 < nplanes && fz_inb(A.err, gz, A.nfield)) qe_next = pmk(A.pi[gz], A.wi[gz]);
-#if !defined(FZ_V_ZAFTER) && !defined(FZ_V_SPLITBAR)
-      // ---- z: centre k+1 -> flux through face k+1/2
-      P vpC;
-      weno_center<R>(qa, qb, qc, qd, qe, vmC, vpC);
-      Fz_hi = godunov<R>(zm, vpC, kA, kC);
-#endif
+      // ---- z: centre k+1
+      weno_waves<R>(qa, qb, qc, qd, qe, A.z0, zr_hi, zl_hi);
     }
 
     // ---- plane k tile
@@ -305,9 +282,6 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
     if (!mbar_wait_bounded(&mbar[buf], parity)) {
       atomicOr(A.err, KERR_TMA_TIMEOUT);
       wait_failed = true;
-#if defined(FZ_V_SPLITBAR)
-      s_abort = 1;
-#endif
     }
     const R* Tp = field(buf, 0);
     const R* Tu = field(buf, 1);
@@ -318,86 +292,53 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
     // after the barrier in one warp-uniform branch, without per-cell tests
     const bool warp_plain = __all_sync(0xffffffffu, valid && ((cls & (CLS_UPDATE | CLS_SOURCE)) == CLS_UPDATE) &&
                                                         !pml_xy && !pml_plane && fz_inb(A.err, gk, A.nfield));
-#if defined(FZ_V_ZAFTER)
-    if (!DIM2) {
-      P vpC;
-      weno_center<R>(qa, qb, qc, qd, qe, vmC, vpC);
-      Fz_hi = godunov<R>(zm, vpC, kA, kC);
-    }
-#endif
 
     // ---- x and y centres of this thread's cell
-    P xm, xp, ym, yp;
+    R xr, xl, yr, yl;
     {
       const int c0 = (ty + HY) * PW + (tx + HX);
-      weno_center<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
-                     pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), xm, xp);
-      XCm[ty * (TX + 2) + tx + 1] = xm;
-      XCp[ty * (TX + 2) + tx + 1] = xp;
-      weno_center<R>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]), pmk(Tp[c0], Tv[c0]),
-                     pmk(Tp[c0 + PW], Tv[c0 + PW]), pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), ym, yp);
-      YCm[(ty + 1) * TX + tx] = ym;
-      YCp[(ty + 1) * TX + tx] = yp;
+      weno_waves<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
+                    pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), A.z0, xr, xl);
+      XR[ty * (TX + 2) + tx + 1] = xr;
+      XL[ty * (TX + 2) + tx + 1] = xl;
+      weno_waves<R>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]), pmk(Tp[c0], Tv[c0]),
+                    pmk(Tp[c0 + PW], Tv[c0 + PW]), pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, yr, yl);
+      YR[(ty + 1) * TX + tx] = yr;
+      YL[(ty + 1) * TX + tx] = yl;
     }
-    // ---- halo centres: warp 0 the x edges (i0-1, i0+TX) of all 16 rows, warps 1-2 the y edge
-    //      rows (j0-1, j0+TY)
+    // ---- halo centres: warp 0 the x edges (wr of i0-1, wl of i0+TX) of all 16 rows, warps 1-2 the
+    //      y edge rows (wr of j0-1, wl of j0+TY)
     if (lt < 2 * TY) {
       const int r = lt >> 1, side = lt & 1;
       const int c0 = (r + HY) * PW + (side ? (HX + TX) : (HX - 1));
-      P em, ep;
-      weno_center<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
-                     pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), em, ep);
-      const int slot = r * (TX + 2) + (side ? TX + 1 : 0);
-      XCm[slot] = em;
-      XCp[slot] = ep;
+      R er, el;
+      weno_waves<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
+                    pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), A.z0, er, el);
+      if (side)
+        XL[r * (TX + 2) + TX + 1] = el;
+      else
+        XR[r * (TX + 2)] = er;
     } else if (lt >= 32 && lt < 32 + 2 * TX) {
       const int e = lt - 32;
       const int c = e & (TX - 1);
-      P em, ep;
-      if constexpr (STAGE == 0 && sizeof(R) == 4 && TX == 32) {  // (16-wide tiles: both rows in one warp)
-        // the fluxes use only V- of row j0-1 and only V+ of row j0+TY (elsewhere the two-branch
-        // form costs the kernel a register spill, so the other instances compute both faces)
-        if (e < TX) {
-          const int c0 = (HY - 1) * PW + (c + HX);
-          weno_center<R, WENO_LO>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
-                                  pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
-                                  pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), em, ep);
-          YCm[c] = em;
-        } else {
-          const int c0 = (TY + HY) * PW + (c + HX);
-          weno_center<R, WENO_HI>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
-                                  pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
-                                  pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), em, ep);
-          YCp[(TY + 1) * TX + c] = ep;
-        }
+      if (e < TX) {
+        const int c0 = (HY - 1) * PW + (c + HX);
+        R er, unused;
+        weno_waves<R, WENO_LO>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
+                               pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
+                               pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, er, unused);
+        YR[c] = er;
       } else {
-        const int r = (e < TX) ? -1 : TY;
-        const int c0 = (r + HY) * PW + (c + HX);
-        weno_center<R>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]), pmk(Tp[c0], Tv[c0]),
-                       pmk(Tp[c0 + PW], Tv[c0 + PW]), pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), em, ep);
-        YCm[(r + 1) * TX + c] = em;
-        YCp[(r + 1) * TX + c] = ep;
+        const int c0 = (TY + HY) * PW + (c + HX);
+        R el, unused;
+        weno_waves<R, WENO_HI>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
+                               pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
+                               pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, unused, el);
+        YL[(TY + 1) * TX + c] = el;
       }
     }
-#if defined(FZ_V_SPLITBAR)
-    // split barrier: each warp arrives once its centres are in shared memory, computes the z centre
-    // (registers only) and only then waits for the other warps' centres
-    __syncwarp();
-    if ((lt & 31) == 0) mbar_arrive(&cbar[it & 1]);
-    if (!DIM2) {
-      P vpC;
-      weno_center<R>(qa, qb, qc, qd, qe, vmC, vpC);
-      Fz_hi = godunov<R>(zm, vpC, kA, kC);
-    }
-    if (!mbar_wait_bounded(&cbar[it & 1], (uint32_t)((it >> 1) & 1))) {
-      atomicOr(A.err, KERR_TMA_TIMEOUT);
-      return;
-    }
-    const bool abort_block = s_abort != 0;
-#else
     // the per-plane barrier, with the OR of the threads' wait failures folded into it
     const bool abort_block = __syncthreads_or(wait_failed) != 0;
-#endif
     if (abort_block) {
 #ifdef FZ_WAIT_TEST
       if (lt == 0) drain_ring(mbar, it, nplanes, A.test_skip_plane);
@@ -412,38 +353,38 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       issue(it + 2);
     }
 
-    // ---- the RK update of this cell before its cPML and source terms: face fluxes and flux
-    //      differences (times h; .x pressure, .y velocity), stage combination
-    auto rk_update = [&](int64_t g, P& Lx, P& Ly, P& Lz, R& pn, R& un, R& vn, R& wn) {
-      Lx = godunov_diff<R>(XCm[ty * (TX + 2) + tx], xp, xm, XCp[ty * (TX + 2) + tx + 2], kA, kC);
-      Ly = godunov_diff<R>(YCm[ty * TX + tx], yp, ym, YCp[(ty + 2) * TX + tx], kA, kC);
-      Lz = psub(Fz_lo, Fz_hi);
-      const R Lp = Lx.x + Ly.x + Lz.x;
+    // ---- the RK update of this cell before its cPML and source terms: per direction the differences
+    //      X of wr and Y of wl across the cell (low minus high face), flux differences (times h)
+    //      c/2 (X - Y) for p and 1/(2 rho) (X + Y) for the velocity; then the stage combination
+    auto rk_update = [&](int64_t g, P& Dx, P& Dy, P& Dz, R& pn, R& un, R& vn, R& wn) {
+      const R Xx = XR[ty * (TX + 2) + tx] - xr, Yx = xl - XL[ty * (TX + 2) + tx + 2];
+      const R Xy = YR[ty * TX + tx] - yr, Yy = yl - YL[(ty + 2) * TX + tx];
+      const R Xz = zr_lo - zr, Yz = zl - zl_hi;
+      Dx = pmk(Xx - Yx, Xx + Yx);
+      Dy = pmk(Xy - Yy, Xy + Yy);
+      Dz = pmk(Xz - Yz, Xz + Yz);
       const int c0 = (ty + HY) * PW + (tx + HX);
-      const R p_in = DIM2 ? Tp[c0] : qb.x, w_in = DIM2 ? A.wi[g] : qb.y;
-      const R u_in = Tu[c0], v_in = Tv[c0];
-      if (STAGE == 0) {
-        pn = p_in + A.dt_h * Lp;
-        un = u_in + A.dt_h * Lx.y;
-        vn = v_in + A.dt_h * Ly.y;
-        wn = w_in + A.dt_h * Lz.y;
-      } else {
+      pn = fma(A.dt_p, (Dx.x + Dy.x) + Dz.x, DIM2 ? Tp[c0] : qb.x);
+      un = fma(A.dt_v, Dx.y, Tu[c0]);
+      vn = fma(A.dt_v, Dy.y, Tv[c0]);
+      wn = fma(A.dt_v, Dz.y, DIM2 ? A.wi[g] : qb.y);
+      if (STAGE > 0) {
         // the stage combination a U0 + b (U_in + dt L) with a + b = 1, written as
         // U0 + b ((U_in + dt L) - U0): the weights sum to one exactly. In FP32 the rounded
         // 1/3 and 2/3 sum to 1 + 3e-8, a gain the whole field would pick up every step (the
         // reference divides by 3 instead, functions3D.cuh:1311-1314, which is unbiased too).
         const R bp = own(buf, 0)[lo], bu = own(buf, 1)[lo], bv = own(buf, 2)[lo], bw = own(buf, 3)[lo];
         const R wb = (STAGE == 1) ? R(0.25) : R(2.0 / 3.0);
-        pn = bp + wb * ((p_in + A.dt_h * Lp) - bp);
-        un = bu + wb * ((u_in + A.dt_h * Lx.y) - bu);
-        vn = bv + wb * ((v_in + A.dt_h * Ly.y) - bv);
-        wn = bw + wb * ((w_in + A.dt_h * Lz.y) - bw);
+        pn = fma(wb, pn - bp, bp);
+        un = fma(wb, un - bu, bu);
+        vn = fma(wb, vn - bv, bv);
+        wn = fma(wb, wn - bw, bw);
       }
     };
     if (warp_plain) {
-      P Lx, Ly, Lz;
+      P Dx, Dy, Dz;
       R pn, un, vn, wn;
-      rk_update(gk, Lx, Ly, Lz, pn, un, vn, wn);
+      rk_update(gk, Dx, Dy, Dz, pn, un, vn, wn);
       A.po[gk] = pn;
       A.uo[gk] = un;
       A.vo[gk] = vn;
@@ -451,9 +392,9 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
     } else if (valid && (cls & (CLS_UPDATE | CLS_SOURCE)) && fz_inb(A.err, gk, A.nfield)) {
       const int64_t g = gk;
       if (cls & CLS_UPDATE) {
-        P Lx, Ly, Lz;
+        P Dx, Dy, Dz;
         R pn, un, vn, wn;
-        rk_update(g, Lx, Ly, Lz, pn, un, vn, wn);
+        rk_update(g, Dx, Dy, Dz, pn, un, vn, wn);
         if (pml_xy || pml_plane) {
           // cPML (functions3D.cuh:725-755): field += w dt ((1/kappa - 1) D + psi), psi frozen
           // within the step and advanced once, in stage 2, by recursive convolution.
@@ -463,7 +404,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
             const int64_t X = cx.tile + d2 * ((int64_t)j + (int64_t)A.Ny * k);
             if (fz_inb(A.err, X, A.npsi[0])) {
             const P ps = A.psix[X];
-            const R Dp = Lx.x * A.inv_h, Du = Lx.y * A.inv_h;
+            const R Dp = Dx.x * A.ih_p, Du = Dx.y * A.ih_v;
             pn += A.wdt * (cx.kinv1 * Dp + ps.x);
             un += A.wdt * (cx.kinv1 * Du + ps.y);
             if (STAGE == 2) A.psix[X] = pmk(cx.b * ps.x + cx.ca * Dp, cx.b * ps.y + cx.ca * Du);
@@ -473,7 +414,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
             const int64_t Y = (int64_t)i + (int64_t)A.Nx * ((int64_t)cy.tile + d2 * k);
             if (fz_inb(A.err, Y, A.npsi[1])) {
             const P ps = A.psiy[Y];
-            const R Dp = Ly.x * A.inv_h, Dv = Ly.y * A.inv_h;
+            const R Dp = Dy.x * A.ih_p, Dv = Dy.y * A.ih_v;
             pn += A.wdt * (cy.kinv1 * Dp + ps.x);
             vn += A.wdt * (cy.kinv1 * Dv + ps.y);
             if (STAGE == 2) A.psiy[Y] = pmk(cy.b * ps.x + cy.ca * Dp, cy.b * ps.y + cy.ca * Dv);
@@ -483,7 +424,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
             const int64_t Z = (int64_t)i + (int64_t)A.Nx * ((int64_t)j + (int64_t)A.Ny * cz.tile);
             if (fz_inb(A.err, Z, A.npsi[2])) {
             const P ps = A.psiz[Z];
-            const R Dp = Lz.x * A.inv_h, Dw = Lz.y * A.inv_h;
+            const R Dp = Dz.x * A.ih_p, Dw = Dz.y * A.ih_v;
             pn += A.wdt * (cz.kinv1 * Dp + ps.x);
             wn += A.wdt * (cz.kinv1 * Dw + ps.y);
             if (STAGE == 2) A.psiz[Z] = pmk(cz.b * ps.x + cz.ca * Dp, cz.b * ps.y + cz.ca * Dw);
@@ -506,8 +447,9 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       buf = 0;
       parity ^= 1u;
     }
-    Fz_lo = Fz_hi;
-    zm = vmC;
+    zr_lo = zr;
+    zr = zr_hi;
+    zl = zl_hi;
     qa = qb;
     qb = qc;
     qc = qd;
