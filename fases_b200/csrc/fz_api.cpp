@@ -81,6 +81,7 @@ void free_device(fz_handle* h) {
   for (auto& p : h->d_pml_coef) dfree(p);
   for (auto& p : h->d_psi) dfree(p);
   dfree(h->d_brec);
+  dfree(h->d_bidx);
   dfree(h->d_bgeo);
   dfree(h->d_bnrm);
   for (auto& set : h->d_ade)
@@ -363,6 +364,23 @@ int build_band(fz_handle* h) {
   return FZ_OK;
 }
 
+// Whether the room runs the direct stage kernel (fz_direct.cu): while its warps, 30 cells of a row
+// each, come to at most two waves of what the GPU holds (16 per SM). Measured, us a step, direct /
+// marching at its best chunk depth: 3D FP32 26 x 22 x 18 (396 warps) 17 / 29, 45 x 38 x 29 (2204) 20 / 33,
+// 71 x 53 x 47 (7473) 49 / 46, 96^3 182 / 93; FP64 18 / 35, 31 / 43, 65 / 65, 283 / 174. A planar room's
+// direct kernel has no redundant centres to pay for, so it goes a little further: FP32 256 x 256 (2304)
+// 18 / 29, 500 x 400 (6800) 36 / 35, FP64 25 / 33, 44 / 50, 800 x 800 (21600) 125 / 113.
+template <class R>
+bool use_direct(const fz_handle* h) {
+#ifdef FZ_WAIT_TEST
+  return false;  // this build is for the marching kernel's bounded waits
+#else
+  const int64_t tiles = (h->Nx - 2 * GHOST + fz::DIRECT_CELLS - 1) / fz::DIRECT_CELLS;
+  const int64_t warps = tiles * (h->Ny - 2 * GHOST) * (h->prm.two_d ? 1 : h->Nz - 2 * GHOST) * h->nb;
+  return warps <= (int64_t)(h->prm.two_d ? 46 : 32) * h->nsm;
+#endif
+}
+
 template <class R>
 int finalize(fz_handle* h) {
   if (h->finalized) return FZ_OK;
@@ -474,6 +492,41 @@ int finalize(fz_handle* h) {
     }
   }
   h->kz_heuristic = (nzi + best - 1) / best;
+  // A room that chunks of 8 planes spread over less than one wave: shallower chunks, by the launch's
+  // latency. In planes of a CTA alone on its SM, a launch takes c0 + sum over waves of (f chunk + c1),
+  // f = 1.45 where two CTAs share the SM; fitted to depths 1 .. 32 of rooms of 10^4 to 10^6 cells
+  // (71 x 53 x 47 FP32: depth 10, the wave model's choice, 84.6 us a step, depth 2 45.9; 64^3 84 -> 47;
+  // FP64 71 x 53 x 47 depth 4 114 -> 65). (Not in the wait-test build, whose hook names a plane of
+  // every chunk.)
+#ifndef FZ_WAIT_TEST
+  if ((int64_t)ntx * nty * h->nb * ((nzi + 7) / 8) <= slots) {
+    const double c0 = occ > 1 ? 1.2 : 2.0, c1 = occ > 1 ? 1.6 : 0.6;
+    double best_t = 1e300;
+    for (int c = 1; c <= nzi; c++) {
+      if (c < (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS) continue;
+      const int64_t items = (int64_t)ntx * nty * h->nb * ((nzi + c - 1) / c);
+      const int64_t full = items / slots, rest = items % slots;
+      const double shared = (occ > 1 ? 1.45 : 1.0) * c + c1;
+      const double t = c0 + full * shared + (rest == 0 ? 0.0 : rest <= h->nsm ? c + c1 : shared);
+      if (t < best_t - 1e-9) {
+        best_t = t;
+        h->kz_heuristic = c;
+      }
+    }
+  }
+#endif
+  h->direct_rule = use_direct<R>(h);
+  if (h->direct_rule && h->nB > 0 && !h->d_bidx) {
+    // band index of every cell, from the band records
+    std::vector<int4> rec((size_t)h->nB);
+    FZ_CUDA(h, cudaMemcpy(rec.data(), h->d_brec, rec.size() * sizeof(int4), cudaMemcpyDeviceToHost), "band D2H");
+    std::vector<int32_t> bidx((size_t)(h->ncell_dev * h->nb), -1);
+    for (size_t b = 0; b < rec.size(); b++)
+      bidx[(size_t)(((uint64_t)(uint32_t)rec[b].y << 32) | (uint32_t)rec[b].x)] = (int32_t)b;
+    FZ_CUDA(h, cudaMalloc(&h->d_bidx, bidx.size() * sizeof(int32_t)), "cudaMalloc(band index)");
+    FZ_CUDA(h, cudaMemcpy(h->d_bidx, bidx.data(), bidx.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
+            "band index H2D");
+  }
   h->finalized = true;
   fzi::set_kz_chunk(h, h->kz_chunk > 0 ? h->kz_chunk : 0);
   return FZ_OK;
@@ -614,10 +667,18 @@ cudaError_t enqueue_stage_kernel(fz_handle* h, int st) {
   return fz::launch_stage<R>(st, h->prm.two_d != 0, stage_args<R>(h, st), m, h->stage_grid, h->stream);
 }
 
-// Stage st of the current step: the stage kernel, then the immersed band (main3D.cu:1286-1306).
+// Stage st of the current step: the stage kernel, then the immersed band (main3D.cu:1286-1306), or
+// both in one launch of the direct kernel.
 template <class R>
 cudaError_t enqueue_stage(fz_handle* h, int st) {
   cudaError_t e;
+  if (h->direct) {
+    Timer t(h, st);
+    const fz::DirectShape sh = fz::direct_shape(h->Nx, h->Ny, h->Nz, h->nb, h->prm.two_d != 0, h->nsm);
+    const fz::DirectArgs d{sh.depth, sh.chunks, h->d_bidx};
+    return fz::launch_stage_direct<R>(st, h->prm.two_d != 0, stage_args<R>(h, st), band_args<R>(h, st), d, sh.grid,
+                                      h->stream);
+  }
   {
     Timer t(h, st);
     e = enqueue_stage_kernel<R>(h, st);
@@ -879,7 +940,7 @@ int bind_field_set(fz_handle* h, int set, void* const* f) {
 cudaError_t enqueue_stage_kernel(fz_handle* h, int st) {
   return h->fp64 ? ::enqueue_stage_kernel<double>(h, st) : ::enqueue_stage_kernel<float>(h, st);
 }
-int set_z_sizes(fz_handle* h, const std::vector<int>& sizes) {
+int set_z_sizes(fz_handle* h, const std::vector<int>& sizes, bool direct) {
   const int nzi = h->Nz - 2 * GHOST;
   int sum = 0;
   for (int c : sizes) {
@@ -893,7 +954,8 @@ int set_z_sizes(fz_handle* h, const std::vector<int>& sizes) {
   const int nty = (h->Ny - 2 * GHOST + fz::TY - 1) / fz::TY;
   const dim3 grid((unsigned)ntx, (unsigned)nty, (unsigned)(sizes.size() * h->nb));
   const bool same = sizes == h->zsizes && grid.x == h->stage_grid.x && grid.y == h->stage_grid.y &&
-                    grid.z == h->stage_grid.z;
+                    grid.z == h->stage_grid.z && h->direct == direct;
+  h->direct = direct;
   h->zsizes = sizes;
   h->zchunks = (int)sizes.size();
   h->kz_chunk = *std::max_element(sizes.begin(), sizes.end());
@@ -914,7 +976,7 @@ void set_kz_chunk(fz_handle* h, int kz_chunk) {
   c = std::max(c, (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS);
   std::vector<int> sizes;
   for (int z = 0; z < nzi; z += c) sizes.push_back(std::min(c, nzi - z));
-  set_z_sizes(h, sizes);
+  set_z_sizes(h, sizes, kz_chunk <= 0 && h->direct_rule);
 }
 
 std::vector<int> guided_z_sizes(fz_handle* h, int depth) {

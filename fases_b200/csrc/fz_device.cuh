@@ -196,6 +196,16 @@ struct BandArgs {
   int64_t nfield;  // elements of one field array (bounds-checked build)
 };
 
+// The direct stage kernel of small rooms (fz_direct.cu): march depth of a warp and chunks of it per
+// member along z, and the band index of every cell (-1: none).
+constexpr int DIRECT_CELLS = 30;  // cells of a row a warp of it updates
+
+struct DirectArgs {
+  int32_t depth;
+  int32_t chunks;
+  const int32_t* bidx;
+};
+
 // Receiver gather of one room (the arguments of its receiver kernel).
 template <class R>
 struct RecArgs {

@@ -117,6 +117,11 @@ struct fz_handle {
   int zchunks = 1;       // z chunks per member
   std::vector<int> zsizes;  // their lengths in planes (sum = interior planes), longest first
   int stage_occ = 1;        // stage-kernel CTAs per SM
+  // the direct stage kernel of small rooms (fz_direct.cu): whether the room's size calls for it,
+  // whether the launches use it now (an explicit tile depth or schedule selects the marching kernel),
+  // and its band index per cell
+  bool direct_rule = false, direct = false;
+  int32_t* d_bidx = nullptr;
   dim3 stage_grid;
 
   // wait-test build: plane of each z chunk whose tile the stage kernels never issue (-1: none)
@@ -168,8 +173,10 @@ cudaError_t enqueue_stage_kernel(fz_handle* h, int st);
 // tile depth of the stage kernels (z planes per CTA; 0 = the wave-filling heuristic); drops the
 // handle's captured graphs
 void set_kz_chunk(fz_handle* h, int kz_chunk);
-// z chunks of any lengths (summing to the interior planes, at most FZ_MAX_ZCHUNKS); drops graphs
-int set_z_sizes(fz_handle* h, const std::vector<int>& sizes);
+// z chunks of any lengths (summing to the interior planes, at most FZ_MAX_ZCHUNKS) of the marching
+// stage kernel, or (direct) the direct kernel with those chunks kept for the shared launches of a
+// group; drops graphs
+int set_z_sizes(fz_handle* h, const std::vector<int>& sizes, bool direct = false);
 // a guided schedule: chunks of `depth` planes, then about one wave of CTAs at depth/2 and one at
 // depth/4, so the last waves are short
 std::vector<int> guided_z_sizes(fz_handle* h, int depth);

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "fz_cell.cuh"
 #include "fz_device.cuh"
 #include "fz_kernels.h"
 #include "fz_pair.cuh"
@@ -110,25 +111,6 @@ struct StageSmem {
 // advance in stage 2 (functions3D.cuh:1157-1162, 1237-1242, 1320-1325), then the point sources of
 // the stage (main3D.cu:1288, 1296, 1304).
 // ------------------------------------------------------------------------------------------
-template <class R>
-__device__ __forceinline__ R source_sum(const StageArgs<R>& A, int64_t g) {
-  const int64_t n = *A.step;
-  const int64_t nn = A.nn_mul * n + A.nn_add;
-  R add = R(0);
-  for (int s = 0; s < A.nsrc; ++s) {
-    if (A.src_cell[s] != g) continue;
-    R amp;
-    if (A.src_opt == 2) {
-      const double ph = 2.0 * 3.14159265358979323846 * (double)A.src_freq[s] * (double)nn * (double)A.half_dt;
-      amp = (R)sin(ph);
-    } else {
-      amp = (nn < A.n_us) ? A.u_s[nn] : R(0);
-    }
-    add += A.src_w * A.src_coef[s] * amp;
-  }
-  return add;
-}
-
 #ifndef FZ_STAGE_MINBLOCKS_F32
 #define FZ_STAGE_MINBLOCKS_F32 (1024 / NTHREADS)  // 32 warps per SM in FP32 (64 registers, no spills)
 #endif
@@ -396,40 +378,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
         R pn, un, vn, wn;
         rk_update(g, Dx, Dy, Dz, pn, un, vn, wn);
         if (pml_xy || pml_plane) {
-          // cPML (functions3D.cuh:725-755): field += w dt ((1/kappa - 1) D + psi), psi frozen
-          // within the step and advanced once, in stage 2, by recursive convolution.
-          const PmlCoef<R> cx = A.pcx[i], cy = A.pcy[j], cz = A.pcz[k];
-          const int64_t d2 = A.pml_d2;
-          if (cx.tile >= 0) {
-            const int64_t X = cx.tile + d2 * ((int64_t)j + (int64_t)A.Ny * k);
-            if (fz_inb(A.err, X, A.npsi[0])) {
-            const P ps = A.psix[X];
-            const R Dp = Dx.x * A.ih_p, Du = Dx.y * A.ih_v;
-            pn += A.wdt * (cx.kinv1 * Dp + ps.x);
-            un += A.wdt * (cx.kinv1 * Du + ps.y);
-            if (STAGE == 2) A.psix[X] = pmk(cx.b * ps.x + cx.ca * Dp, cx.b * ps.y + cx.ca * Du);
-            }
-          }
-          if (cy.tile >= 0) {
-            const int64_t Y = (int64_t)i + (int64_t)A.Nx * ((int64_t)cy.tile + d2 * k);
-            if (fz_inb(A.err, Y, A.npsi[1])) {
-            const P ps = A.psiy[Y];
-            const R Dp = Dy.x * A.ih_p, Dv = Dy.y * A.ih_v;
-            pn += A.wdt * (cy.kinv1 * Dp + ps.x);
-            vn += A.wdt * (cy.kinv1 * Dv + ps.y);
-            if (STAGE == 2) A.psiy[Y] = pmk(cy.b * ps.x + cy.ca * Dp, cy.b * ps.y + cy.ca * Dv);
-            }
-          }
-          if (cz.tile >= 0) {
-            const int64_t Z = (int64_t)i + (int64_t)A.Nx * ((int64_t)j + (int64_t)A.Ny * cz.tile);
-            if (fz_inb(A.err, Z, A.npsi[2])) {
-            const P ps = A.psiz[Z];
-            const R Dp = Dz.x * A.ih_p, Dw = Dz.y * A.ih_v;
-            pn += A.wdt * (cz.kinv1 * Dp + ps.x);
-            wn += A.wdt * (cz.kinv1 * Dw + ps.y);
-            if (STAGE == 2) A.psiz[Z] = pmk(cz.b * ps.x + cz.ca * Dp, cz.b * ps.y + cz.ca * Dw);
-            }
-          }
+          pml_update<R, STAGE>(A, i, j, k, A.pcx[i], A.pcy[j], A.pcz[k], Dx, Dy, Dz, pn, un, vn, wn);
         }
         if (cls & CLS_SOURCE) pn += source_sum(A, g);
         A.po[g] = pn;
@@ -463,153 +412,20 @@ __global__ void __launch_bounds__(NTHREADS, sizeof(R) == 4 ? FZ_STAGE_MINBLOCKS_
   stage_body<R, STAGE, DIM2, GridCta>(A, M);
 }
 
-// ------------------------------------------------------------------------------------------
-// Immersed ADE band (functions3D.cuh:462-565 + ADE_solver 426-459), one thread per band cell of
-// the compact list. Probe geometry (normal, trilinear corner and weights at C - 2h n, chi) is
-// precomputed once on the host. The probe reads the stage-input fields, which no kernel of this
-// stage writes; the blend reads and writes only the band cell itself.
-// ------------------------------------------------------------------------------------------
-template <class R>
-__device__ __forceinline__ R trilin(const R* __restrict__ f, int64_t q, int64_t Sx, int64_t plane, R sx,
-                                    R sy, R sz) {
-  const R c00 = __ldg(f + q) * (R(1) - sx) + __ldg(f + q + 1) * sx;
-  const R c10 = __ldg(f + q + Sx) * (R(1) - sx) + __ldg(f + q + Sx + 1) * sx;
-  const R c01 = __ldg(f + q + plane) * (R(1) - sx) + __ldg(f + q + plane + 1) * sx;
-  const R c11 = __ldg(f + q + plane + Sx) * (R(1) - sx) + __ldg(f + q + plane + Sx + 1) * sx;
-  const R c0 = c00 * (R(1) - sy) + c10 * sy, c1 = c01 * (R(1) - sy) + c11 * sy;
-  return c0 * (R(1) - sz) + c1 * sz;
-}
-
-template <class R>
-struct Vec4;
-template <>
-struct Vec4<float> {
-  typedef float4 T;
-};
-template <>
-struct Vec4<double> {
-  typedef double4 T;
-};
-
-// STAGE selects the ADE stage coefficients (a, b, c) = (0,1,1), (3,1,4), (1,2,3)
-// (main3D.cu:1290, 1298, 1306): left = (a middle + b (right + dt L(right))) / c.
-// KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
-// probe (the cell's own fields, the ADE states of the stage) is then issued at the top, beside the
-// probe gathers, so one thread keeps ~50 loads in flight; KM = LM = 0 is the general form with
-// the state loads inside the pole loops.
+// One band cell of the separate band kernels: its stage output (written by the stage kernel) is
+// loaded beside the probe and blended in place.
 template <class R, int STAGE, int KM, int LM>
 __device__ __forceinline__ void band_body(const BandArgs<R>& B, const int64_t b) {
-  typedef typename Vec4<R>::T V4;
   if (b >= B.nB) return;
   const int4 rc = __ldg(B.rec + b);
   const int64_t cell = (int64_t)(((uint64_t)(uint32_t)rc.y << 32) | (uint32_t)rc.x);
-  const int64_t q = cell + rc.z;
-  const int m = rc.w;
-  const int64_t nB = B.nB;
-  if (!fz_inb(B.err, cell, B.nfield) || !fz_inb(B.err, q, B.nfield) ||
-      !fz_inb(B.err, q + B.plane + B.Sx + 1, B.nfield))
-    return;
-  const V4 g4 = reinterpret_cast<const V4*>(B.geo)[b];
-  const V4 n4 = reinterpret_cast<const V4*>(B.nrm)[b];
-  // the cell's own stage output (written by the stage kernel, blended here by this thread only)
-  R po0 = R(0), uo0 = R(0), vo0 = R(0), wo0 = R(0);
-  if (KM > 0) {
-    po0 = B.po[cell];
-    uo0 = B.uo[cell];
-    vo0 = B.vo[cell];
-    wo0 = B.wo[cell];
-  }
-  double rK[KM > 0 ? KM : 1], mK[KM > 0 ? KM : 1], r1L[LM > 0 ? LM : 1], r2L[LM > 0 ? LM : 1];
-  double m1L[LM > 0 ? LM : 1], m2L[LM > 0 ? LM : 1];
-#pragma unroll
-  for (int k = 0; k < KM; ++k)
-    if (k < B.K) {
-      rK[k] = __ldg(B.phR + (int64_t)k * nB + b);
-      if (STAGE > 0) mK[k] = __ldg(B.phM + (int64_t)k * nB + b);
-    }
-#pragma unroll
-  for (int l = 0; l < LM; ++l)
-    if (l < B.L) {
-      r1L[l] = __ldg(B.s1R + (int64_t)l * nB + b);
-      r2L[l] = __ldg(B.s2R + (int64_t)l * nB + b);
-      if (STAGE > 0) {
-        m1L[l] = __ldg(B.s1M + (int64_t)l * nB + b);
-        m2L[l] = __ldg(B.s2M + (int64_t)l * nB + b);
-      }
-    }
-  const R sx = g4.x, sy = g4.y, sz = g4.z, chi = g4.w;
-  const R nx = n4.x, ny = n4.y, nz = n4.z;
-  const R pD = trilin<R>(B.pi, q, B.Sx, B.plane, sx, sy, sz);
-  const R uD = trilin<R>(B.ui, q, B.Sx, B.plane, sx, sy, sz);
-  const R vD = trilin<R>(B.vi, q, B.Sx, B.plane, sx, sy, sz);
-  const R wD = trilin<R>(B.wi, q, B.Sx, B.plane, sx, sy, sz);
-  const R un = uD * nx + vD * ny + wD * nz;
-  const R utx = uD - un * nx, uty = vD - un * ny, utz = wD - un * nz;
-  const double wout = (double)pD + B.Z0 * (double)un;  // outgoing characteristic
-  constexpr double a_ssp = (STAGE == 0) ? 0.0 : (STAGE == 1) ? 3.0 : 1.0;
-  constexpr double b_ssp = (STAGE == 2) ? 2.0 : 1.0;
-  constexpr double inv_c = (STAGE == 0) ? 1.0 : (STAGE == 1) ? 0.25 : 1.0 / 3.0;
-  double sumA = 0.0, sumBC = 0.0;
-  // one real pole / complex pair of the ADE stage recursion
-  auto real_pole = [&](int k, double r, double mid) {
-    const int mi = m * B.K + k;
-    const double Lphi = wout - __ldg(B.zeta + mi) * r;
-    double v = b_ssp * (r + B.dt * Lphi);
-    if (STAGE > 0) v += a_ssp * mid;
-    v *= inv_c;
-    B.phL[(int64_t)k * nB + b] = v;
-    sumA += __ldg(B.A + mi) * v;
-  };
-  auto pole_pair = [&](int l, double r1, double r2, double m1, double m2) {
-    const int mi = m * B.L + l;
-    const double al = __ldg(B.alpha + mi), be = __ldg(B.beta + mi);
-    const double L1 = wout - (al * r1 + be * r2);
-    const double L2 = be * r1 - al * r2;
-    double n1 = b_ssp * (r1 + B.dt * L1);
-    double n2 = b_ssp * (r2 + B.dt * L2);
-    if (STAGE > 0) {
-      n1 += a_ssp * m1;
-      n2 += a_ssp * m2;
-    }
-    n1 *= inv_c;
-    n2 *= inv_c;
-    const int64_t si = (int64_t)l * nB + b;
-    B.s1L[si] = n1;
-    B.s2L[si] = n2;
-    sumBC += __ldg(B.B + mi) * n1 + __ldg(B.C + mi) * n2;
-  };
-  if constexpr (KM > 0) {
-#pragma unroll
-    for (int k = 0; k < KM; ++k)
-      if (k < B.K) real_pole(k, rK[k], STAGE > 0 ? mK[k] : 0.0);
-#pragma unroll
-    for (int l = 0; l < LM; ++l)
-      if (l < B.L) pole_pair(l, r1L[l], r2L[l], STAGE > 0 ? m1L[l] : 0.0, STAGE > 0 ? m2L[l] : 0.0);
-  } else {
-    for (int k = 0; k < B.K; ++k) {
-      const int64_t si = (int64_t)k * nB + b;
-      real_pole(k, B.phR[si], STAGE > 0 ? B.phM[si] : 0.0);
-    }
-    for (int l = 0; l < B.L; ++l) {
-      const int64_t si = (int64_t)l * nB + b;
-      pole_pair(l, B.s1R[si], B.s2R[si], STAGE > 0 ? B.s1M[si] : 0.0, STAGE > 0 ? B.s2M[si] : 0.0);
-    }
-  }
-  const double win = __ldg(B.Rinf + m) * wout + sumA + sumBC;  // incoming characteristic
-  const R pb = (R)(0.5 * (win + wout));
-  const R unb = (R)((wout - win) / (2.0 * B.Z0));
-  const R ub = unb * nx + utx, vb = unb * ny + uty, wb = unb * nz + utz;
-  const R omc = R(1) - chi;
-  if (KM == 0) {
-    po0 = B.po[cell];
-    uo0 = B.uo[cell];
-    vo0 = B.vo[cell];
-    wo0 = B.wo[cell];
-  }
-  B.uo[cell] = omc * uo0 + chi * ub;
-  B.vo[cell] = omc * vo0 + chi * vb;
-  B.wo[cell] = omc * wo0 + chi * wb;
-  B.po[cell] = omc * po0 + chi * pb;
+  if (!band_inb(B, cell, rc)) return;
+  R p = B.po[cell], u = B.uo[cell], v = B.vo[cell], w = B.wo[cell];
+  band_cell<R, STAGE, KM, LM>(B, b, cell, rc, p, u, v, w);
+  B.uo[cell] = u;
+  B.vo[cell] = v;
+  B.wo[cell] = w;
+  B.po[cell] = p;
 }
 
 #define FZ_BAND_BOUNDS(R, KM) __launch_bounds__(256, (sizeof(R) == 4 && KM > 0 && KM <= 2) ? 4 : 3)

@@ -16,6 +16,15 @@ cudaError_t stage_occupancy(int* blocks_per_sm);
 template <class R>
 cudaError_t launch_stage(int stage, bool two_d, const StageArgs<R>& a, const StageMaps& m, dim3 grid,
                          cudaStream_t s);
+// the direct stage kernel of small rooms: launch shape for a room, and the launch (stage and band)
+struct DirectShape {
+  int depth, chunks;
+  dim3 grid;
+};
+DirectShape direct_shape(int Nx, int Ny, int Nz, int nb, bool two_d, int nsm);
+template <class R>
+cudaError_t launch_stage_direct(int stage, bool two_d, const StageArgs<R>& a, const BandArgs<R>& b,
+                                const DirectArgs& d, dim3 grid, cudaStream_t s);
 template <class R>
 cudaError_t launch_band(int stage, const BandArgs<R>& a, cudaStream_t s);
 template <class R>

@@ -91,7 +91,7 @@ std::vector<ZPlan> kz_candidates(fz_handle* h) {
   const int nzi = h->Nz - 2 * GHOST;
   std::vector<ZPlan> out{{0, 0}};
   if (nzi <= 1) return out;
-  // every distinct depth ceil(nzi / nk) of at least 4 planes, ranked by the heuristic's model
+  // every distinct depth ceil(nzi / nk) of at least 2 planes, ranked by the heuristic's model
   const int occ = std::max(1, h->stage_occ);
   const int ntx = (h->Nx - 2 * GHOST + fz::TX - 1) / fz::TX;
   const int nty = (h->Ny - 2 * GHOST + fz::TY - 1) / fz::TY;
@@ -100,7 +100,7 @@ std::vector<ZPlan> kz_candidates(fz_handle* h) {
   int last = -1;
   for (int nk = 1; nk <= nzi; nk++) {
     const int c = (nzi + nk - 1) / nk;
-    if (c < 4) break;
+    if (c < 2) break;
     if (c == last) continue;
     last = c;
     const int64_t items = (int64_t)ntx * nty * ((nzi + c - 1) / c) * h->nb;
@@ -151,7 +151,9 @@ int tune(const std::vector<fz_handle*>& hs, cudaStream_t ts, const std::vector<Z
       fz_handle* h = hs[q];
       if (h->stream != ts) x = cudaStreamWaitEvent(h->stream, fork, 0);
       for (int r = 0; r < n && x == cudaSuccess; r++)
-        for (int st = 0; st < 3 && x == cudaSuccess; st++) x = enqueue_stage_kernel(h, st);
+        for (int st = 0; st < 3 && x == cudaSuccess; st++)
+          // the direct kernel includes the band: against it, the others are timed with theirs
+          x = h->direct_rule ? enqueue_stage(h, st) : enqueue_stage_kernel(h, st);
       if (x == cudaSuccess && h->stream != ts) x = cudaEventRecord(join[q], h->stream);
       if (x == cudaSuccess && h->stream != ts) x = cudaStreamWaitEvent(ts, join[q], 0);
     }
