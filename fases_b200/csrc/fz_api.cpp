@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "fz_internal.h"
+#include "fz_wait.h"
 #include "fz_kernels.h"
 
 using fz::XOFF;
@@ -1583,7 +1584,6 @@ int fz_sync(fz_handle* h, int64_t timeout_ms) {
   if (timeout_ms <= 0) timeout_ms = 600000;
   cudaSetDevice(h->device);
   const auto t0 = std::chrono::steady_clock::now();
-  int sleep_us = 20;
   for (;;) {
     cudaError_t e = cudaStreamQuery(h->stream);
     if (e == cudaSuccess) {
@@ -1606,8 +1606,7 @@ int fz_sync(fz_handle* h, int64_t timeout_ms) {
     const auto ms =
         std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
     if (ms > timeout_ms) return set_error(h, FZ_ETIMEOUT, "fz_sync: device work did not finish in time");
-    std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-    sleep_us = std::min(sleep_us * 2, 2000);
+    fz::poll_pause(t0);
   }
 }
 

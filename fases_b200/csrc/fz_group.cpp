@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "fz_internal.h"
+#include "fz_wait.h"
 #include "fz_kernels.h"
 
 // Launch arguments of every member for one buffer-parity key. Device memory holds [3 stages][n]
@@ -602,7 +603,6 @@ int fz_group_sync(fz_group* g, int64_t timeout_ms) {
   if (timeout_ms <= 0) timeout_ms = 600000;
   cudaSetDevice(g->device);
   const auto t0 = std::chrono::steady_clock::now();
-  int sleep_us = 20;
   for (;;) {
     const cudaError_t e = cudaStreamQuery(g->stream);
     if (e == cudaSuccess) break;
@@ -610,8 +610,7 @@ int fz_group_sync(fz_group* g, int64_t timeout_ms) {
     const auto ms =
         std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
     if (ms > timeout_ms) return fzi::set_global_error(FZ_ETIMEOUT, "fz_group_sync: device work did not finish in time");
-    std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-    sleep_us = std::min(sleep_us * 2, 2000);
+    fz::poll_pause(t0);
   }
   for (fz_handle* h : g->m) {  // each member's own stream and device error word
     const int rc = fz_sync(h, timeout_ms);

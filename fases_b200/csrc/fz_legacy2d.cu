@@ -30,6 +30,7 @@
 
 #include "fz.h"
 #include "fz_legacy2d.h"
+#include "fz_wait.h"
 
 namespace l2d {
 
@@ -436,15 +437,13 @@ int build_band(fz_l2d* h, const float* S, const uint8_t* oid, std::vector<int32_
 
 int wait(fz_l2d* h) {
   const auto t0 = std::chrono::steady_clock::now();
-  int sleep_us = 20;
   for (;;) {
     const cudaError_t e = cudaStreamQuery(h->stream);
     if (e == cudaSuccess) break;
     if (e != cudaErrorNotReady) return cuda_fail(h, e, "stream");
     if (std::chrono::steady_clock::now() - t0 > std::chrono::minutes(10))
       return fail(h, FZ_ETIMEOUT, "fz_l2d: device work did not finish in time");
-    std::this_thread::sleep_for(std::chrono::microseconds(sleep_us));
-    sleep_us = std::min(sleep_us * 2, 2000);
+    fz::poll_pause(t0);
   }
   int32_t kerr = 0;
   L2D_CUDA(h, cudaMemcpy(&kerr, h->d_err, sizeof(kerr), cudaMemcpyDeviceToHost), "error word D2H");
