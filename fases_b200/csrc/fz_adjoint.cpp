@@ -160,6 +160,7 @@ int misfit_gradient(fz_handle* h, int64_t nsteps, int seg, const double* target,
   for (int r = 0; r < 3; r++)
     for (int a = 0; a < 3; a++) own_ade[r][a] = h->d_ade[r][a];
   auto unbind = [&]() -> int {
+    h->keep_ade = false;
     for (int r = 0; r < 3; r++)
       for (int a = 0; a < 3; a++) h->d_ade[r][a] = own_ade[r][a];
     for (int q = 0; q < 3; q++) {
@@ -359,6 +360,7 @@ int misfit_gradient(fz_handle* h, int64_t nsteps, int seg, const double* target,
       for (int a = 0; a < 3; a++) h->d_ade[role][a] = Ad[q][a][(size_t)t];
     };
     point_ade(h->ph_old, 0, 0);
+    h->keep_ade = true;  // the sweep reads the states after every stage
     for (int t = 0; t < len; t++) {
       cudaError_t e = cudaSuccess;
       for (int a = 0; a < 3 && e == cudaSuccess && want_pml; a++)

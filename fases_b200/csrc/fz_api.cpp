@@ -83,6 +83,7 @@ void free_device(fz_handle* h) {
   for (auto& p : h->d_psi) dfree(p);
   dfree(h->d_brec);
   dfree(h->d_bidx);
+  dfree(h->d_wst);
   dfree(h->d_bgeo);
   dfree(h->d_bnrm);
   for (auto& set : h->d_ade)
@@ -409,6 +410,7 @@ int finalize(fz_handle* h) {
   FZ_CUDA(h, cudaMemcpy(h->d_mat, packed.data(), packed.size() * 8, cudaMemcpyHostToDevice), "materials H2D");
   // ADE states (3 rotating sets, main3D.cu:683-709), zeroed
   if (h->nB > 0) {
+    FZ_CUDA(h, cudaMalloc(&h->d_wst, (size_t)h->nB * 2 * 8), "cudaMalloc(ADE)");
     const size_t nk = (size_t)h->nB * h->K, nl = (size_t)h->nB * h->L;
     for (int s = 0; s < 3; s++) {
       FZ_CUDA(h, cudaMalloc(&h->d_ade[s][0], nk * 8), "cudaMalloc(ADE)");
@@ -623,6 +625,8 @@ fz::BandArgs<R> band_args(fz_handle* h, int stage) {
   b.phL = h->d_ade[L_][0]; b.phM = h->d_ade[M_][0]; b.phR = h->d_ade[R_][0];
   b.s1L = h->d_ade[L_][1]; b.s1M = h->d_ade[M_][1]; b.s1R = h->d_ade[R_][1];
   b.s2L = h->d_ade[L_][2]; b.s2M = h->d_ade[M_][2]; b.s2R = h->d_ade[R_][2];
+  b.wst = h->d_wst;
+  b.keep = h->keep_ade ? 1 : 0;
   b.K = h->K; b.L = h->L;
   const int nm = std::max(1, h->nMat);
   const double* m = h->d_mat;

@@ -96,13 +96,40 @@ __device__ __forceinline__ bool band_inb(const BandArgs<R>& B, int64_t cell, con
          fz_inb(B.err, cell + rc.z + B.plane + B.Sx + 1, B.nfield);
 }
 
-// STAGE selects the ADE stage coefficients (a, b, c) = (0,1,1), (3,1,4), (1,2,3)
-// (main3D.cu:1290, 1298, 1306): left = (a middle + b (right + dt L(right))) / c.
+// One pole state of an ADE stage, left = (a middle + b (right + dt L(right))) / c with the stage's
+// (a, b, c) = (0,1,1), (3,1,4), (1,2,3) (main3D.cu:1290, 1298, 1306), given the rate L(right).
+template <int STAGE>
+__device__ __forceinline__ double ade_advance(double right, double rate, double mid, double dt) {
+  constexpr double a = (STAGE == 0) ? 0.0 : (STAGE == 1) ? 3.0 : 1.0;
+  constexpr double b = (STAGE == 2) ? 2.0 : 1.0;
+  constexpr double inv_c = (STAGE == 0) ? 1.0 : (STAGE == 1) ? 0.25 : 1.0 / 3.0;
+  double x = b * fma(dt, rate, right);
+  if (STAGE > 0) x = fma(a, mid, x);
+  return x * inv_c;
+}
+template <int STAGE>
+__device__ __forceinline__ double ade_real(double right, double mid, double zeta, double wout, double dt) {
+  return ade_advance<STAGE>(right, fma(-zeta, right, wout), mid, dt);
+}
+template <int STAGE>
+__device__ __forceinline__ void ade_pair(double& r1, double& r2, double m1, double m2, double al, double be,
+                                         double wout, double dt) {
+  const double n1 = ade_advance<STAGE>(r1, wout - fma(al, r1, be * r2), m1, dt);
+  r2 = ade_advance<STAGE>(r2, fma(be, r1, -(al * r2)), m2, dt);
+  r1 = n1;
+}
+
+// The band cell b at `cell`: (p, u, v, w) is the cell's stage output on entry, the blended values on
+// return.
+// KEEP: the pole states after this stage are stored (the left role), and the stage reads its right and
+// middle sets. Otherwise only the last stage stores states: the recursion is linear in the state at
+// step start and the outgoing characteristics, so stages 1 and 2 recompute the earlier stages' states
+// from those (8 bytes a stage, kept in wst) instead of reading and writing sets of 8 (K + 2L) bytes.
+// With K = L = 2 a band cell moves 176 instead of 384 bytes of states a step, with the same bits.
 // KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
-// probe (the ADE states of the stage) is then issued at the top, beside the probe gathers, so one
-// thread keeps ~50 loads in flight; KM = LM = 0 is the general form with the state loads inside the
-// pole loops. (p, u, v, w): the cell's stage output on entry, the blended values on return.
-template <class R, int STAGE, int KM, int LM>
+// probe is then issued at the top, beside the probe gathers, so one thread keeps ~50 loads in flight;
+// KM = LM = 0 is the general form with the state loads inside the pole loops.
+template <class R, int STAGE, int KM, int LM, bool KEEP>
 __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b, const int64_t cell, const int4& rc,
                                           R& p, R& u, R& v, R& w) {
   typedef typename Vec4<R>::T V4;
@@ -111,24 +138,28 @@ __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b,
   const int64_t nB = B.nB;
   const V4 g4 = reinterpret_cast<const V4*>(B.geo)[b];
   const V4 n4 = reinterpret_cast<const V4*>(B.nrm)[b];
+  constexpr bool RIGHT = KEEP && STAGE > 0;  // the right set is not the step-start (middle) one
   double rK[KM > 0 ? KM : 1], mK[KM > 0 ? KM : 1], r1L[LM > 0 ? LM : 1], r2L[LM > 0 ? LM : 1];
   double m1L[LM > 0 ? LM : 1], m2L[LM > 0 ? LM : 1];
 #pragma unroll
   for (int k = 0; k < KM; ++k)
     if (k < B.K) {
-      rK[k] = __ldg(B.phR + (int64_t)k * nB + b);
-      if (STAGE > 0) mK[k] = __ldg(B.phM + (int64_t)k * nB + b);
+      mK[k] = __ldg(B.phM + (int64_t)k * nB + b);
+      if (RIGHT) rK[k] = __ldg(B.phR + (int64_t)k * nB + b);
     }
 #pragma unroll
   for (int l = 0; l < LM; ++l)
     if (l < B.L) {
-      r1L[l] = __ldg(B.s1R + (int64_t)l * nB + b);
-      r2L[l] = __ldg(B.s2R + (int64_t)l * nB + b);
-      if (STAGE > 0) {
-        m1L[l] = __ldg(B.s1M + (int64_t)l * nB + b);
-        m2L[l] = __ldg(B.s2M + (int64_t)l * nB + b);
+      m1L[l] = __ldg(B.s1M + (int64_t)l * nB + b);
+      m2L[l] = __ldg(B.s2M + (int64_t)l * nB + b);
+      if (RIGHT) {
+        r1L[l] = __ldg(B.s1R + (int64_t)l * nB + b);
+        r2L[l] = __ldg(B.s2R + (int64_t)l * nB + b);
       }
     }
+  double w0 = 0.0, w1 = 0.0;  // the outgoing characteristics of the earlier stages
+  if (!KEEP && STAGE > 0) w0 = __ldg(B.wst + b);
+  if (!KEEP && STAGE > 1) w1 = __ldg(B.wst + nB + b);
   const R sx = g4.x, sy = g4.y, sz = g4.z, chi = g4.w;
   const R nx = n4.x, ny = n4.y, nz = n4.z;
   const R pD = trilin<R>(B.pi, q, B.Sx, B.plane, sx, sy, sz);
@@ -138,48 +169,51 @@ __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b,
   const R un = fma(wD, nz, fma(vD, ny, uD * nx));
   const R utx = fma(-un, nx, uD), uty = fma(-un, ny, vD), utz = fma(-un, nz, wD);
   const double wout = fma(B.Z0, (double)un, (double)pD);  // outgoing characteristic
-  constexpr double a_ssp = (STAGE == 0) ? 0.0 : (STAGE == 1) ? 3.0 : 1.0;
-  constexpr double b_ssp = (STAGE == 2) ? 2.0 : 1.0;
-  constexpr double inv_c = (STAGE == 0) ? 1.0 : (STAGE == 1) ? 0.25 : 1.0 / 3.0;
+  if (!KEEP && STAGE < 2) B.wst[STAGE * nB + b] = wout;
   const double dt = B.dt;
-  // one pole state of the ADE stage recursion: (a mid + b (r + dt L)) / c
-  auto advance = [&](double r, double rate, double mid) {
-    double x = b_ssp * fma(dt, rate, r);
-    if (STAGE > 0) x = fma(a_ssp, mid, x);
-    return x * inv_c;
-  };
   double sumA = 0.0, sumBC = 0.0;
   auto real_pole = [&](int k, double r, double mid) {
     const int mi = m * B.K + k;
-    const double x = advance(r, fma(-__ldg(B.zeta + mi), r, wout), mid);
-    B.phL[(int64_t)k * nB + b] = x;
-    sumA = fma(__ldg(B.A + mi), x, sumA);
+    const double zeta = __ldg(B.zeta + mi);
+    if (!RIGHT) r = mid;
+    if (!KEEP && STAGE > 0) r = ade_real<0>(r, mid, zeta, w0, dt);
+    if (!KEEP && STAGE > 1) r = ade_real<1>(r, mid, zeta, w1, dt);
+    r = ade_real<STAGE>(r, mid, zeta, wout, dt);
+    if (KEEP || STAGE == 2) B.phL[(int64_t)k * nB + b] = r;
+    sumA = fma(__ldg(B.A + mi), r, sumA);
   };
   auto pole_pair = [&](int l, double r1, double r2, double m1, double m2) {
     const int mi = m * B.L + l;
     const double al = __ldg(B.alpha + mi), be = __ldg(B.beta + mi);
-    const double n1 = advance(r1, wout - fma(al, r1, be * r2), m1);
-    const double n2 = advance(r2, fma(be, r1, -(al * r2)), m2);
+    if (!RIGHT) {
+      r1 = m1;
+      r2 = m2;
+    }
+    if (!KEEP && STAGE > 0) ade_pair<0>(r1, r2, m1, m2, al, be, w0, dt);
+    if (!KEEP && STAGE > 1) ade_pair<1>(r1, r2, m1, m2, al, be, w1, dt);
+    ade_pair<STAGE>(r1, r2, m1, m2, al, be, wout, dt);
     const int64_t si = (int64_t)l * nB + b;
-    B.s1L[si] = n1;
-    B.s2L[si] = n2;
-    sumBC = fma(__ldg(B.B + mi), n1, fma(__ldg(B.C + mi), n2, sumBC));
+    if (KEEP || STAGE == 2) {
+      B.s1L[si] = r1;
+      B.s2L[si] = r2;
+    }
+    sumBC = fma(__ldg(B.B + mi), r1, fma(__ldg(B.C + mi), r2, sumBC));
   };
   if constexpr (KM > 0) {
 #pragma unroll
     for (int k = 0; k < KM; ++k)
-      if (k < B.K) real_pole(k, rK[k], STAGE > 0 ? mK[k] : 0.0);
+      if (k < B.K) real_pole(k, rK[k], mK[k]);
 #pragma unroll
     for (int l = 0; l < LM; ++l)
-      if (l < B.L) pole_pair(l, r1L[l], r2L[l], STAGE > 0 ? m1L[l] : 0.0, STAGE > 0 ? m2L[l] : 0.0);
+      if (l < B.L) pole_pair(l, r1L[l], r2L[l], m1L[l], m2L[l]);
   } else {
     for (int k = 0; k < B.K; ++k) {
       const int64_t si = (int64_t)k * nB + b;
-      real_pole(k, B.phR[si], STAGE > 0 ? B.phM[si] : 0.0);
+      real_pole(k, RIGHT ? B.phR[si] : 0.0, B.phM[si]);
     }
     for (int l = 0; l < B.L; ++l) {
       const int64_t si = (int64_t)l * nB + b;
-      pole_pair(l, B.s1R[si], B.s2R[si], STAGE > 0 ? B.s1M[si] : 0.0, STAGE > 0 ? B.s2M[si] : 0.0);
+      pole_pair(l, RIGHT ? B.s1R[si] : 0.0, RIGHT ? B.s2R[si] : 0.0, B.s1M[si], B.s2M[si]);
     }
   }
   const double win = fma(__ldg(B.Rinf + m), wout, sumA + sumBC);  // incoming characteristic

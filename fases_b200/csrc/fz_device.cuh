@@ -192,6 +192,8 @@ struct BandArgs {
   double* s2L;
   const double* s2M;
   const double* s2R;
+  double* wst;     // [2*nB]: outgoing characteristics of stages 0 and 1 of the current step
+  int32_t keep;    // the states after every stage are wanted (the adjoint's recompute)
   int32_t* err;    // device error word (bounds-checked build)
   int64_t nfield;  // elements of one field array (bounds-checked build)
 };

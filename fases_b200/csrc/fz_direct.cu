@@ -148,7 +148,7 @@ __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArg
         }
       }
       if (KM >= 0 && b >= 0 && band_inb(B, g, rc))
-        band_cell<R, STAGE, KM < 0 ? 0 : KM, LM>(B, b, g, rc, pn, un, vn, wn);
+        band_cell<R, STAGE, KM < 0 ? 0 : KM, LM, true>(B, b, g, rc, pn, un, vn, wn);
       A.po[g] = pn;
       if ((cls & CLS_UPDATE) || (KM >= 0 && b >= 0)) {
         A.uo[g] = un;

@@ -65,6 +65,8 @@ struct fz_handle {
   void* d_bnrm = nullptr;
   double* d_ade[3][3] = {{nullptr}};  // [set][phi, psi1, psi2]
   int ph_old = 0, ph_cur = 1, ph_nu = 2;
+  double* d_wst = nullptr;  // outgoing characteristics of stages 0 and 1 of a step, per band record
+  bool keep_ade = false;    // the band kernels store the states after every stage (the adjoint's recompute)
 
   // materials
   int nMat = 0, K = 1, L = 1;

@@ -414,14 +414,14 @@ __global__ void __launch_bounds__(NTHREADS, sizeof(R) == 4 ? FZ_STAGE_MINBLOCKS_
 
 // One band cell of the separate band kernels: its stage output (written by the stage kernel) is
 // loaded beside the probe and blended in place.
-template <class R, int STAGE, int KM, int LM>
+template <class R, int STAGE, int KM, int LM, bool KEEP>
 __device__ __forceinline__ void band_body(const BandArgs<R>& B, const int64_t b) {
   if (b >= B.nB) return;
   const int4 rc = __ldg(B.rec + b);
   const int64_t cell = (int64_t)(((uint64_t)(uint32_t)rc.y << 32) | (uint32_t)rc.x);
   if (!band_inb(B, cell, rc)) return;
   R p = B.po[cell], u = B.uo[cell], v = B.vo[cell], w = B.wo[cell];
-  band_cell<R, STAGE, KM, LM>(B, b, cell, rc, p, u, v, w);
+  band_cell<R, STAGE, KM, LM, KEEP>(B, b, cell, rc, p, u, v, w);
   B.uo[cell] = u;
   B.vo[cell] = v;
   B.wo[cell] = w;
@@ -430,9 +430,9 @@ __device__ __forceinline__ void band_body(const BandArgs<R>& B, const int64_t b)
 
 #define FZ_BAND_BOUNDS(R, KM) __launch_bounds__(256, (sizeof(R) == 4 && KM > 0 && KM <= 2) ? 4 : 3)
 
-template <class R, int STAGE, int KM, int LM>
+template <class R, int STAGE, int KM, int LM, bool KEEP>
 __global__ void FZ_BAND_BOUNDS(R, KM) k_band(const __grid_constant__ BandArgs<R> B) {
-  band_body<R, STAGE, KM, LM>(B, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  band_body<R, STAGE, KM, LM, KEEP>(B, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Receiver gather after the last stage of a step (main3D.cu:1399-1414), into a device buffer;
@@ -523,7 +523,7 @@ __global__ void FZ_BAND_BOUNDS(R, KM) k_band_group(const __grid_constant__ Group
   const int m = group_member(G.blk_start, G.n, blockIdx.x);
   copy_args(sB, G.args + m, threadIdx.x, blockDim.x);
   __syncthreads();
-  band_body<R, STAGE, KM, LM>(sB, (int64_t)((int)blockIdx.x - G.blk_start[m]) * blockDim.x + threadIdx.x);
+  band_body<R, STAGE, KM, LM, false>(sB, (int64_t)((int)blockIdx.x - G.blk_start[m]) * blockDim.x + threadIdx.x);
 }
 
 // one block per member
@@ -702,19 +702,19 @@ cudaError_t launch_band(int stage, const BandArgs<R>& a, cudaStream_t s) {
   const int64_t nb = (a.nB + bs - 1) / bs;
   // pole counts of up to 2 (4) real poles and complex pairs take the fixed-size form
   const int fit = (a.K <= 2 && a.L <= 2) ? 2 : (a.K <= 4 && a.L <= 4) ? 4 : 0;
-#define FZ_BAND_LAUNCH(ST)                                                    \
+#define FZ_BAND_LAUNCH(ST, KEEP)                                              \
   if (fit == 2)                                                               \
-    k_band<R, ST, 2, 2><<<(unsigned)nb, bs, 0, s>>>(a);                       \
+    k_band<R, ST, 2, 2, KEEP><<<(unsigned)nb, bs, 0, s>>>(a);                 \
   else if (fit == 4)                                                          \
-    k_band<R, ST, 4, 4><<<(unsigned)nb, bs, 0, s>>>(a);                       \
+    k_band<R, ST, 4, 4, KEEP><<<(unsigned)nb, bs, 0, s>>>(a);                 \
   else                                                                        \
-    k_band<R, ST, 0, 0><<<(unsigned)nb, bs, 0, s>>>(a);
+    k_band<R, ST, 0, 0, KEEP><<<(unsigned)nb, bs, 0, s>>>(a);
   if (stage == 0) {
-    FZ_BAND_LAUNCH(0)
+    if (a.keep) { FZ_BAND_LAUNCH(0, true) } else { FZ_BAND_LAUNCH(0, false) }
   } else if (stage == 1) {
-    FZ_BAND_LAUNCH(1)
+    if (a.keep) { FZ_BAND_LAUNCH(1, true) } else { FZ_BAND_LAUNCH(1, false) }
   } else {
-    FZ_BAND_LAUNCH(2)
+    if (a.keep) { FZ_BAND_LAUNCH(2, true) } else { FZ_BAND_LAUNCH(2, false) }
   }
 #undef FZ_BAND_LAUNCH
   return cudaGetLastError();

@@ -72,21 +72,52 @@ __device__ __forceinline__ typename Pair<R>::T psplat(R x) {
 // caller uses one of them (the tile's halo rows); the value computed is the same either way.
 constexpr int WENO_LO = 1, WENO_HI = 2, WENO_BOTH = 3;
 
-// The weighted sums and normalisers of a centre: V- = q0 + Nm / Sm, V+ = q0 - Np / Sp.
-template <int FACES>
-__device__ __forceinline__ void weno_sums(float2 qm2, float2 qm1, float2 q0, float2 qp1, float2 qp2, float2& Nm,
-                                          float2& Np, float2& rSm, float2& rSp) {
+// Nonlinear weights from the indicators B_r = 3/4 (beta_r + eps), up to a factor common to the three
+// (it cancels between the sums and their normalisers).
+struct WenoZ {  // 1 + tau / B_r, tau = |B_0 - B_2|
+  __device__ __forceinline__ void operator()(float2 B0, float2 B1, float2 B2, float2& w0, float2& w1, float2& w2) const {
+    const float2 tau = pabs(psub(B0, B2)), one = make_float2(1.f, 1.f);
+    w0 = pfma(tau, prcp(B0), one);
+    w1 = pfma(tau, prcp(B1), one);
+    w2 = pfma(tau, prcp(B2), one);
+  }
+  // In FP64 a reciprocal costs several FMA-pipe operations: the factors times B_0 B_1 B_2
+  __device__ __forceinline__ void operator()(double B0, double B1, double B2, double& w0, double& w1, double& w2) const {
+    const double tau = fabs(B0 - B2);
+    const double B12 = B1 * B2, B02 = B0 * B2, B01 = B0 * B1, B012 = B0 * B12;
+    w0 = fma(tau, B12, B012);
+    w1 = fma(tau, B02, B012);
+    w2 = fma(tau, B01, B012);
+  }
+};
+struct WenoJS {  // 1 / B_r^2 (Jiang & Shu 1996)
+  __device__ __forceinline__ void operator()(float2 B0, float2 B1, float2 B2, float2& w0, float2& w1, float2& w2) const {
+    const float2 r0 = prcp(B0), r1 = prcp(B1), r2 = prcp(B2);
+    w0 = pmul(r0, r0);
+    w1 = pmul(r1, r1);
+    w2 = pmul(r2, r2);
+  }
+  __device__ __forceinline__ void operator()(double B0, double B1, double B2, double& w0, double& w1, double& w2) const {
+    const double B12 = B1 * B2, B02 = B0 * B2, B01 = B0 * B1;
+    w0 = B12 * B12;
+    w1 = B02 * B02;
+    w2 = B01 * B01;
+  }
+};
+
+// The weighted sums and normalisers of a centre: V- = q0 + Nm / Sm, V+ = q0 - Np / Sp. eps: 3/4 of the
+// scheme's.
+template <int FACES, class W>
+__device__ __forceinline__ void weno_sums(float2 qm2, float2 qm1, float2 q0, float2 qp1, float2 qp2, float eps,
+                                          W weights, float2& Nm, float2& Np, float2& rSm, float2& rSp) {
   auto K = [](float x) { return make_float2(x, x); };
-  constexpr float eps = 0.75e-10f;
   const float2 a = psub(qm1, qm2), b = psub(q0, qm1), c = psub(qp1, q0), d = psub(qp2, qp1);
   const float2 bb = pfma(b, b, K(eps));
   const float2 B1 = pfma(c, pfma(b, K(-1.25f), c), bb);
   const float2 B2 = pfma(a, pfma(b, K(-2.75f), a), pfma(bb, K(2.5f), K(-1.5f * eps)));
   const float2 B0 = pfma(d, pfma(c, K(-2.75f), d), pfma(pmul(c, K(2.5f)), c, K(eps)));
-  const float2 tau = pabs(psub(B0, B2));
-  const float2 w0 = pfma(tau, prcp(B0), K(1.f));
-  const float2 w1 = pfma(tau, prcp(B1), K(1.f));
-  const float2 w2 = pfma(tau, prcp(B2), K(1.f));
+  float2 w0, w1, w2;
+  weights(B0, B1, B2, w0, w1, w2);
   const float2 t1 = pmul(w1, K(3.f));
   if constexpr ((FACES & WENO_LO) != 0) {
     rSm = prcp(pfma(w0, K(1.5f), pfma(w2, K(0.5f), t1)));
@@ -112,25 +143,20 @@ __device__ __forceinline__ double drcp(double x) {
   return fma(r, fma(e, e, e), r);
 }
 
-// In FP64 a reciprocal costs several FMA-pipe operations, so the factors 1 + tau / B_r are taken
-// times B_0 B_1 B_2 (the common factor cancels between N and S) and both normalisers share one
-// reciprocal: 1 instead of 5 per variable (190 x 150 x 140 cells: a stage 0.175-0.183 ms instead of
-// 0.265-0.272). B lies in [eps, amplitude^2], so the products (up to
-// B^7) stay inside the double range for amplitudes below 1e20.
-template <int FACES>
-__device__ __forceinline__ void weno_sums1(double qm2, double qm1, double q0, double qp1, double qp2, double& Nm,
-                                           double& Np, double& rSm, double& rSp) {
-  constexpr double eps = 0.75e-10;
+// In FP64 the weights come without reciprocals (above) and both normalisers share one: 1 instead of 5
+// per variable (190 x 150 x 140 cells: a stage 0.175-0.183 ms instead of 0.265-0.272). B lies in
+// [eps, amplitude^2], so the products (up to B^8) stay inside the double range for amplitudes below
+// 1e18.
+template <int FACES, class W>
+__device__ __forceinline__ void weno_sums1(double qm2, double qm1, double q0, double qp1, double qp2, double eps,
+                                           W weights, double& Nm, double& Np, double& rSm, double& rSp) {
   const double a = qm1 - qm2, b = q0 - qm1, c = qp1 - q0, d = qp2 - qp1;
   const double bb = fma(b, b, eps);
   const double B1 = fma(c, fma(b, -1.25, c), bb);
   const double B2 = fma(a, fma(b, -2.75, a), fma(bb, 2.5, -1.5 * eps));
   const double B0 = fma(d, fma(c, -2.75, d), fma(2.5 * c, c, eps));
-  const double tau = fabs(B0 - B2);
-  const double B12 = B1 * B2, B02 = B0 * B2, B01 = B0 * B1, B012 = B0 * B12;
-  const double w0 = fma(tau, B12, B012);
-  const double w1 = fma(tau, B02, B012);
-  const double w2 = fma(tau, B01, B012);
+  double w0, w1, w2;
+  weights(B0, B1, B2, w0, w1, w2);
   const double t1 = 3.0 * w1;
   const double Sm = fma(w0, 1.5, fma(w2, 0.5, t1)), Sp = fma(w0, 0.5, fma(w2, 1.5, t1));
   const double r = drcp(Sm * Sp);
@@ -145,11 +171,11 @@ __device__ __forceinline__ void weno_sums1(double qm2, double qm1, double q0, do
     Np = fma(w2, g2, fma(w1, g1, w0 * g0));
   }
 }
-template <int FACES>
-__device__ __forceinline__ void weno_sums(double2 qm2, double2 qm1, double2 q0, double2 qp1, double2 qp2, double2& Nm,
-                                          double2& Np, double2& rSm, double2& rSp) {
-  weno_sums1<FACES>(qm2.x, qm1.x, q0.x, qp1.x, qp2.x, Nm.x, Np.x, rSm.x, rSp.x);
-  weno_sums1<FACES>(qm2.y, qm1.y, q0.y, qp1.y, qp2.y, Nm.y, Np.y, rSm.y, rSp.y);
+template <int FACES, class W>
+__device__ __forceinline__ void weno_sums(double2 qm2, double2 qm1, double2 q0, double2 qp1, double2 qp2, double eps,
+                                          W weights, double2& Nm, double2& Np, double2& rSm, double2& rSp) {
+  weno_sums1<FACES>(qm2.x, qm1.x, q0.x, qp1.x, qp2.x, eps, weights, Nm.x, Np.x, rSm.x, rSp.x);
+  weno_sums1<FACES>(qm2.y, qm1.y, q0.y, qp1.y, qp2.y, eps, weights, Nm.y, Np.y, rSm.y, rSp.y);
 }
 
 // Outgoing characteristics of a centre, all the Godunov flux needs of it (functions3D.cuh:56-78 with
@@ -157,11 +183,12 @@ __device__ __forceinline__ void weno_sums(double2 qm2, double2 qm1, double2 q0, 
 // left-going one at the face below, wl = p - Z0 q of V+(i-1/2). The flux through a face is
 //   F_p = c/2 (wr(i) - wl(i+1)),   F_q = 1/(2 rho) (wr(i) + wl(i+1)),
 // so centres exchange two numbers instead of four.
-template <class R, int FACES = WENO_BOTH>
+template <class R, int FACES = WENO_BOTH, class W = WenoZ>
 __device__ __forceinline__ void weno_waves(typename Pair<R>::T qm2, typename Pair<R>::T qm1, typename Pair<R>::T q0,
-                                           typename Pair<R>::T qp1, typename Pair<R>::T qp2, R Z0, R& wr, R& wl) {
+                                           typename Pair<R>::T qp1, typename Pair<R>::T qp2, R Z0, R& wr, R& wl,
+                                           R eps = R(0.75e-10)) {
   typename Pair<R>::T Nm, Np, rm, rp;
-  weno_sums<FACES>(qm2, qm1, q0, qp1, qp2, Nm, Np, rm, rp);
+  weno_sums<FACES>(qm2, qm1, q0, qp1, qp2, eps, W(), Nm, Np, rm, rp);
   if constexpr ((FACES & WENO_LO) != 0) wr = fma(Z0, fma(Nm.y, rm.y, q0.y), fma(Nm.x, rm.x, q0.x));
   if constexpr ((FACES & WENO_HI) != 0) wl = fma(-Z0, fma(-Np.y, rp.y, q0.y), fma(-Np.x, rp.x, q0.x));
 }
@@ -171,7 +198,7 @@ __device__ __forceinline__ void weno_center(typename Pair<R>::T qm2, typename Pa
                                             typename Pair<R>::T qp1, typename Pair<R>::T qp2, typename Pair<R>::T& vm,
                                             typename Pair<R>::T& vp) {
   typename Pair<R>::T Nm, Np, rm, rp;
-  weno_sums<WENO_BOTH>(qm2, qm1, q0, qp1, qp2, Nm, Np, rm, rp);
+  weno_sums<WENO_BOTH>(qm2, qm1, q0, qp1, qp2, R(0.75e-10), WenoZ(), Nm, Np, rm, rp);
   vm = pfma(Nm, rm, q0);
   vp = psub(q0, pmul(Np, rp));
 }
