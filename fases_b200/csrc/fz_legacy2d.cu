@@ -30,6 +30,7 @@
 
 #include "fz.h"
 #include "fz_legacy2d.h"
+#include "fz_pair.cuh"
 #include "fz_wait.h"
 
 namespace l2d {
@@ -51,8 +52,10 @@ struct Band {
 template <class R>
 struct Args {
   int Nx, Ny;
-  R h, dt, rho, c, eps;
-  R keyN, keyS, keyE, keyW, half;
+  R rho, c, dt;
+  R eps;         // 3/4 of the scheme's (fz_pair.cuh)
+  R dt_p, dt_v;  // dt / h * c / 2, dt / h / (2 rho): per difference / sum of the characteristics
+  const R *spx, *spy;  // sPML ramps along x and y
   const R* in[3];    // stage input p, u, v (stencils and probes)
   const R* base[3];  // U0 p, u, v (stages 1 and 2)
   R* out[3];
@@ -73,36 +76,16 @@ struct Args {
   int32_t* err;
 };
 
-// WENO5-JS value at face i+1/2 (IDX 1) or i-1/2 (IDX 0) of the node f points at, stride st;
-// candidate and smoothness tables of 2D-solver/core/main.cu:638-651, weights of
-// functions.cuh:1096-1112, the smoothness indicator in double as functions.cuh:1115-1123
-template <class R, int IDX>
-__device__ __forceinline__ R weno_js(const R* f, int st, R eps) {
-  constexpr double crl[4][3] = {{11.0 / 6.0, -7.0 / 6.0, 1.0 / 3.0},
-                                {1.0 / 3.0, 5.0 / 6.0, -1.0 / 6.0},
-                                {-1.0 / 6.0, 5.0 / 6.0, 1.0 / 3.0},
-                                {1.0 / 3.0, -7.0 / 6.0, 11.0 / 6.0}};
-  constexpr double brl[3][3] = {{3, -4, 1}, {1, 0, -1}, {1, -4, 3}};
-  constexpr double dd[3] = {3.0 / 10.0, 3.0 / 5.0, 1.0 / 10.0};
-  R V[3], al[3];
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    const R q0 = f[-r * st], q1 = f[(1 - r) * st], q2 = f[(2 - r) * st];
-    R acc = R(0);
-    acc += (R)crl[r + IDX][0] * q0;
-    acc += (R)crl[r + IDX][1] * q1;
-    acc += (R)crl[r + IDX][2] * q2;
-    V[r] = acc;
-    const R b1 = q0 - R(2) * q1 + q2;
-    const R b2 = (R)brl[r][0] * q0 + (R)brl[r][1] * q1 + (R)brl[r][2] * q2;
-    const R bt = (R)((13.0 * (double)b1 * (double)b1 / 12.0) + (0.25 * (double)b2 * (double)b2));
-    const R aux = bt + eps;
-    al[r] = (R)dd[IDX == 1 ? r : 2 - r] / (aux * aux);
-  }
-  R out = R(0);
-#pragma unroll
-  for (int r = 0; r < 3; r++) out += (al[r] / (al[0] + al[1] + al[2])) * V[r];
-  return out;
+// WENO5-JS centre (candidate and smoothness tables of 2D-solver/core/main.cu:638-651, weights of
+// functions.cuh:1096-1123) for the pair (p, normal velocity): the characteristics its two faces hand to
+// the Godunov flux, as fz_pair.cuh evaluates them for the 3D scheme. The indicators are quadratic forms
+// of first differences, which are exact where the field is smooth; the reference forms second
+// differences from the values themselves (rounding at the size of p) and squares those in double.
+template <class R>
+__device__ __forceinline__ void js_waves(const R* fp, const R* fv, int st, R eps, R Z0, R& wr, R& wl) {
+  fz::weno_waves<R, fz::WENO_BOTH, fz::WenoJS>(fz::pmk(fp[-2 * st], fv[-2 * st]), fz::pmk(fp[-st], fv[-st]),
+                                               fz::pmk(fp[0], fv[0]), fz::pmk(fp[st], fv[st]),
+                                               fz::pmk(fp[2 * st], fv[2 * st]), Z0, wr, wl, eps);
 }
 
 template <class R>
@@ -118,8 +101,8 @@ __device__ __forceinline__ R cubic(R fm1, R f0, R f1, R f2, R s) {
 template <class R, int STAGE>
 __global__ void __launch_bounds__(NT) k_l2d_stage(const Args<R> a) {
   __shared__ R sm[3][SY][SX];
-  __shared__ R xf[4][TY][FX];  // p+, p-, u+, u- of nodes i0-1 .. i0+TX
-  __shared__ R yf[4][FY][TX];  // p+, p-, v+, v- of nodes j0-1 .. j0+TY
+  __shared__ R xw[2][TY][FX];  // characteristics (right-going, left-going) of nodes i0-1 .. i0+TX
+  __shared__ R yw[2][FY][TX];  // of nodes j0-1 .. j0+TY
   const int t = threadIdx.x;
   const int i0 = blockIdx.x * TX + HALO, j0 = blockIdx.y * TY + HALO;
   for (int q = t; q < SX * SY; q += NT) {
@@ -131,88 +114,53 @@ __global__ void __launch_bounds__(NT) k_l2d_stage(const Args<R> a) {
     for (int f = 0; f < 3; f++) sm[f][y][x] = ok ? a.in[f][g] : R(0);
   }
   __syncthreads();
-  // face values: WENO_x / WENO_y of functions.cuh:1125-1176, each face once
+  // this thread's own node, its loads issued before the centres
+  const int tx = t % TX, ty = t / TX;
+  const int i = i0 + tx, j = j0 + ty;
+  const bool mine = t < TX * TY && i < a.Nx - 3 && j < a.Ny - 3;
+  const size_t C = (size_t)j * a.Nx + i;
+  const uint8_t cl = mine ? a.cls[C] : (uint8_t)0;
+  R b0 = R(0), b1 = R(0), b2 = R(0);
+  if (STAGE > 0 && (cl & FLUID)) {
+    b0 = a.base[0][C];
+    b1 = a.base[1][C];
+    b2 = a.base[2][C];
+  }
+  // centres: each once (WENO_x / WENO_y of functions.cuh:1125-1176)
+  const R Z0 = a.rho * a.c;
   if (t < FX * TY) {
     const int row = t / FX, col = t % FX;  // node (i0 + col - 1, j0 + row)
-    const R* fp = &sm[0][row + HALO][col + HALO - 1];
-    const R* fu = &sm[1][row + HALO][col + HALO - 1];
-    xf[0][row][col] = weno_js<R, 1>(fp, 1, a.eps);
-    xf[1][row][col] = weno_js<R, 0>(fp, 1, a.eps);
-    xf[2][row][col] = weno_js<R, 1>(fu, 1, a.eps);
-    xf[3][row][col] = weno_js<R, 0>(fu, 1, a.eps);
+    js_waves<R>(&sm[0][row + HALO][col + HALO - 1], &sm[1][row + HALO][col + HALO - 1], 1, a.eps, Z0, xw[0][row][col],
+                xw[1][row][col]);
   }
   {
     const int row = t / TX, col = t % TX;  // node (i0 + col, j0 + row - 1)
-    const R* fp = &sm[0][row + HALO - 1][col + HALO];
-    const R* fv = &sm[2][row + HALO - 1][col + HALO];
-    yf[0][row][col] = weno_js<R, 1>(fp, SX, a.eps);
-    yf[1][row][col] = weno_js<R, 0>(fp, SX, a.eps);
-    yf[2][row][col] = weno_js<R, 1>(fv, SX, a.eps);
-    yf[3][row][col] = weno_js<R, 0>(fv, SX, a.eps);
+    js_waves<R>(&sm[0][row + HALO - 1][col + HALO], &sm[2][row + HALO - 1][col + HALO], SX, a.eps, Z0, yw[0][row][col],
+                yw[1][row][col]);
   }
   __syncthreads();
-  if (t >= TX * TY) return;
-  const int tx = t % TX, ty = t / TX;
-  const int i = i0 + tx, j = j0 + ty;
-  if (i >= a.Nx - 3 || j >= a.Ny - 3) return;
-  const size_t C = (size_t)j * a.Nx + i;
-  const uint8_t cl = a.cls[C];
+  if (!mine) return;
   R np, nu, nv;
   if (cl & FLUID) {
     const R* sp = &sm[0][ty + HALO][tx + HALO];
     const R* su = &sm[1][ty + HALO][tx + HALO];
     const R* sv = &sm[2][ty + HALO][tx + HALO];
-    const R rho = a.rho, c = a.c;
-    // Godunov fluxes of functions.cuh:199-213 (the 0.5 applied in double as there) on the face
-    // values of compute_Vs_x / compute_Vs_y: [0] V+ at i, [1] V- at i+1, [2] V+ at i-1, [3] V- at i
-    auto Fp = [&](R pM, R pP, R uM, R uP) { return (R)(0.5 * (double)(rho * c * c * (uP + uM) - c * (pP - pM))); };
-    auto Fu = [&](R pM, R pP, R uM, R uP) { return (R)(0.5 * (double)((pP + pM) / rho - c * (uP - uM))); };
-    auto Gv = [&](R pM, R pP, R vM, R vP) { return (R)(0.5 * (double)((pM + pP) / rho - c * (vP - vM))); };
-    R FpP, FpM, FuP, FuM, GpP, GpM, GvP, GvM;
-    {
-      const int x = tx + 1;
-      const R p0 = xf[0][ty][x], p1 = xf[1][ty][x + 1], p2 = xf[0][ty][x - 1], p3 = xf[1][ty][x];
-      const R u0 = xf[2][ty][x], u1 = xf[3][ty][x + 1], u2 = xf[2][ty][x - 1], u3 = xf[3][ty][x];
-      FpP = Fp(p0, p1, u0, u1);
-      FpM = Fp(p2, p3, u2, u3);
-      FuP = Fu(p0, p1, u0, u1);
-      FuM = Fu(p2, p3, u2, u3);
-    }
-    {
-      const int y = ty + 1;
-      const R p0 = yf[0][y][tx], p1 = yf[1][y + 1][tx], p2 = yf[0][y - 1][tx], p3 = yf[1][y][tx];
-      const R v0 = yf[2][y][tx], v1 = yf[3][y + 1][tx], v2 = yf[2][y - 1][tx], v3 = yf[3][y][tx];
-      GpP = Fp(p0, p1, v0, v1);
-      GpM = Fp(p2, p3, v2, v3);
-      GvP = Gv(p0, p1, v0, v1);
-      GvM = Gv(p2, p3, v2, v3);
-    }
-    const R ru = a.dt * ((-FuP + FuM) / a.h);
-    const R rv = a.dt * ((-GvP + GvM) / a.h);
-    const R rp = a.dt * ((-FpP + FpM - GpP + GpM) / a.h);
-    // kernel_WENO_step0/1/2 combinations (functions.cuh:1241-1243, 1311-1313, 1378-1380)
-    if (STAGE == 0) {
-      nu = *su + ru;
-      nv = *sv + rv;
-      np = *sp + rp;
-    } else if (STAGE == 1) {
-      nu = (R)0.75f * a.base[1][C] + (R)0.25f * (*su + ru);
-      nv = (R)0.75f * a.base[2][C] + (R)0.25f * (*sv + rv);
-      np = (R)0.75f * a.base[0][C] + (R)0.25f * (*sp + rp);
-    } else {
-      nu = (a.base[1][C] + R(2) * (*su + ru)) / R(3);
-      nv = (a.base[2][C] + R(2) * (*sv + rv)) / R(3);
-      np = (a.base[0][C] + R(2) * (*sp + rp)) / R(3);
+    // Godunov fluxes of functions.cuh:199-213 on the characteristics: per direction the differences X
+    // of the right-going and Y of the left-going ones across the node (low minus high face)
+    const R Xx = xw[0][ty][tx] - xw[0][ty][tx + 1], Yx = xw[1][ty][tx + 1] - xw[1][ty][tx + 2];
+    const R Xy = yw[0][ty][tx] - yw[0][ty + 1][tx], Yy = yw[1][ty + 1][tx] - yw[1][ty + 2][tx];
+    np = fma(a.dt_p, (Xx - Yx) + (Xy - Yy), *sp);
+    nu = fma(a.dt_v, Xx + Yx, *su);
+    nv = fma(a.dt_v, Xy + Yy, *sv);
+    // kernel_WENO_step1/2 combinations (functions.cuh:1311-1313, 1378-1380), their weights summing to one
+    if (STAGE > 0) {
+      const R wb = (STAGE == 1) ? R(0.25) : R(2.0 / 3.0);
+      np = fma(wb, np - b0, b0);
+      nu = fma(wb, nu - b1, b1);
+      nv = fma(wb, nv - b2, b2);
     }
     // sPML (functions.cuh:941-965)
-    const R one = R(1), zero = R(0), half = a.half;
-    const R rx = a.keyE * fmax(zero, fmin((R)(i - (a.Nx - half)) / half, one));
-    const R lx = a.keyW * fmax(zero, fmin((half - i) / half, one));
-    const R ly = a.keyS * fmax(zero, fmin((half - j) / half, one));
-    const R uy = a.keyN * fmax(zero, fmin((j - (a.Ny - half)) / half, one));
-    const R smax = (R)0.018f;
-    const R sx = smax * (rx * rx * rx + lx * lx * lx);
-    const R sy = smax * (uy * uy * uy + ly * ly * ly);
+    const R sx = a.spx[i], sy = a.spy[j];
     const R s = fmin(sx + sy - sx * sy, (R)0.999f);
     nu -= s * nu;
     nv -= s * nv;
@@ -264,7 +212,6 @@ __global__ void __launch_bounds__(NT) k_l2d_stage(const Args<R> a) {
     const R nx = g.nx, ny = g.ny;
     const R un = uD * nx + vD * ny;
     const R ut = -uD * ny + vD * nx;
-    const R Z0 = a.rho * a.c;
     const R w_out = pD + Z0 * un;
     // ADE_solver (functions.cuh:635-669)
     const int m = g.mat;
@@ -322,6 +269,7 @@ struct fz_l2d {
   size_t N = 0;
   bool fp64 = false;
   void* buf[3][3] = {};      // [buffer][p,u,v]; buffers 0/1 swap the U0/U1 roles, 2 is U2
+  void* d_sp[2] = {};        // sPML ramps along x and y
   uint8_t* d_cls = nullptr;
   uint8_t* d_colfluid = nullptr;
   int32_t* d_bidx = nullptr;
@@ -451,14 +399,36 @@ int wait(fz_l2d* h) {
   return FZ_OK;
 }
 
+// sPML ramps of functions.cuh:941-965 along an axis of N nodes, in the arithmetic of the field type
+// (evaluated once here instead of per node and stage)
+template <class R>
+cudaError_t upload_spml(fz_l2d* h, int axis) {
+  const fz_l2d_params& p = h->prm;
+  const int N = axis == 0 ? p.Nx : p.Ny;
+  const R lo = (R)(axis == 0 ? p.pml_w : p.pml_s), hi = (R)(axis == 0 ? p.pml_e : p.pml_n);
+  const R half = (R)(int)(0.15f * (float)std::min(p.Nx, p.Ny)), one = R(1), zero = R(0);
+  std::vector<R> s((size_t)N);
+  for (int i = 0; i < N; i++) {
+    const R r = hi * std::max(zero, std::min((R)(i - (N - half)) / half, one));
+    const R l = lo * std::max(zero, std::min((half - i) / half, one));
+    s[(size_t)i] = (R)0.018f * (r * r * r + l * l * l);
+  }
+  cudaError_t e = cudaMalloc(&h->d_sp[axis], s.size() * sizeof(R));
+  if (e == cudaSuccess) e = cudaMemcpy(h->d_sp[axis], s.data(), s.size() * sizeof(R), cudaMemcpyHostToDevice);
+  return e;
+}
+
 template <class R>
 l2d::Args<R> args(fz_l2d* h, int stage, int par) {
   l2d::Args<R> a{};
   const fz_l2d_params& p = h->prm;
   a.Nx = p.Nx; a.Ny = p.Ny;
-  a.h = (R)p.h; a.dt = (R)p.dt; a.rho = (R)p.rho; a.c = (R)p.c; a.eps = (R)p.eps;
-  a.keyN = (R)p.pml_n; a.keyS = (R)p.pml_s; a.keyE = (R)p.pml_e; a.keyW = (R)p.pml_w;
-  a.half = (R)(int)(0.15f * (float)std::min(p.Nx, p.Ny));
+  a.dt = (R)p.dt; a.rho = (R)p.rho; a.c = (R)p.c;
+  a.eps = (R)(0.75 * p.eps);
+  a.dt_p = (R)(0.5 * p.dt * p.c / p.h);
+  a.dt_v = (R)(0.5 * p.dt / (p.h * p.rho));
+  a.spx = (const R*)h->d_sp[0];
+  a.spy = (const R*)h->d_sp[1];
   const int b0 = par, b1 = 1 - par;
   const int in = stage == 0 ? b0 : (stage == 1 ? b1 : 2);
   const int out = stage == 1 ? 2 : b1;
@@ -573,6 +543,8 @@ int fz_l2d_create(const fz_l2d_params* p, fz_l2d** out) {
     for (int f = 0; f < 3; f++)
       if (bad(cudaMalloc(&h->buf[b][f], h->N * rsize(h))) || bad(cudaMemset(h->buf[b][f], 0, h->N * rsize(h))))
         return FZ_ENOMEM;
+  for (int axis = 0; axis < 2; axis++)
+    if (bad(h->fp64 ? upload_spml<double>(h, axis) : upload_spml<float>(h, axis))) return FZ_ENOMEM;
   if (bad(cudaMalloc(&h->d_step, sizeof(int64_t))) || bad(cudaMemset(h->d_step, 0, sizeof(int64_t))) ||
       bad(cudaMalloc(&h->d_err, sizeof(int32_t))) || bad(cudaMemset(h->d_err, 0, sizeof(int32_t))))
     return FZ_ENOMEM;
@@ -590,6 +562,7 @@ int fz_l2d_destroy(fz_l2d* h) {
   for (auto& q : h->d_state)
     for (void*& s : q) cudaFree(s);
   for (void*& c : h->d_coef) cudaFree(c);
+  for (void*& c : h->d_sp) cudaFree(c);
   cudaFree(h->d_cls); cudaFree(h->d_colfluid); cudaFree(h->d_bidx); cudaFree(h->d_band);
   cudaFree(h->d_ir); cudaFree(h->d_step); cudaFree(h->d_err);
   if (h->stream) cudaStreamDestroy(h->stream);
