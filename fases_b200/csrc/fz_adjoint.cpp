@@ -288,7 +288,7 @@ int misfit_gradient(fz_handle* h, int64_t nsteps, int seg, const double* target,
   const int64_t slots = (int64_t)h->nsm * occ;
   int best = 1;
   double best_eff = -1.0;
-  for (int nk = 1; nk <= std::max(1, nzi / 8); nk++) {
+  for (int nk = 1; nk <= std::max(1, nzi / 2); nk++) {
     const int chunk = (nzi + nk - 1) / nk;
     const int64_t items = (int64_t)ntx * nty * ((nzi + chunk - 1) / chunk);
     const int64_t waves = (items + slots - 1) / slots;

@@ -9,89 +9,102 @@
 #include <algorithm>
 
 #include "fz_adjoint.h"
+#include "fz_cell.cuh"
 #include "fz_pair.cuh"
 
 namespace fz {
 
 namespace {
 
+// Reciprocals of the three indicators and of the two normalisers. In FP64 a reciprocal costs several
+// FMA-pipe operations, so each group shares one.
+__device__ __forceinline__ void rcp3(float2 a, float2 b, float2 c, float2& ra, float2& rb, float2& rc) {
+  ra = prcp(a);
+  rb = prcp(b);
+  rc = prcp(c);
+}
+__device__ __forceinline__ void rcp3(double a, double b, double c, double& ra, double& rb, double& rc) {
+  const double bc = b * c, r = drcp(a * bc), t = r * a;
+  ra = r * bc;
+  rb = t * c;
+  rc = t * b;
+}
+__device__ __forceinline__ void rcp3(double2 a, double2 b, double2 c, double2& ra, double2& rb, double2& rc) {
+  rcp3(a.x, b.x, c.x, ra.x, rb.x, rc.x);
+  rcp3(a.y, b.y, c.y, ra.y, rb.y, rc.y);
+}
+__device__ __forceinline__ void rcp2(float2 a, float2 b, float2& ra, float2& rb) {
+  ra = prcp(a);
+  rb = prcp(b);
+}
+__device__ __forceinline__ void rcp2(double2 a, double2 b, double2& ra, double2& rb) {
+  const double x = drcp(a.x * b.x), y = drcp(a.y * b.y);
+  ra = make_double2(x * b.x, y * b.y);
+  rb = make_double2(x * a.x, y * a.y);
+}
+
 // Reverse mode of one WENO-Z cell centre for a pair of variables (pressure and the velocity
 // component along the sweep): u[0..4] are the values at c-2 .. c+2; the centre gives V-(c+1/2)
 // (lam_m, its adjoint) and V+(c-1/2) (lam_p) from one set of smoothness indicators, as the
-// stepping kernels' weno_core computes them (first differences a..d, second differences D_r,
-// E_r, 12/13-scaled indicators B_r, q_r = 1 + tau/B_r, normalisers Sm, Sp). g[0..4] += lam_m
-// dV-/du + lam_p dV+/du. The forward part is recomputed; reciprocals are differentiated as exact
-// 1/x. tau = |B0 - B2| takes the subgradient sign(0) = 0.
+// stepping kernels' weno_sums computes them (first differences a..d, indicators B_r as quadratic
+// forms of them, w_r = 1 + tau/B_r, V- = u + Nm/Sm, V+ = u - Np/Sp). g[0..4] += lam_m dV-/du + lam_p
+// dV+/du. The forward part is recomputed; reciprocals are differentiated as exact 1/x. tau =
+// |B0 - B2| takes the subgradient sign(0) = 0. 107 paired operations and 5 (FP64: 2) reciprocals,
+// where the sweep back through second differences took 128 and 5.
 template <class R>
 __device__ __forceinline__ void weno_centre_rev(const typename Pair<R>::T u[5], typename Pair<R>::T lam_m,
                                                 typename Pair<R>::T lam_p, typename Pair<R>::T g[5]) {
   typedef typename Pair<R>::T P;
   auto K = [](double x) { return psplat<R>(R(x)); };
-  // ---- forward (weno_core)
+  constexpr double eps = 0.75e-10, k512 = 5.0 / 12.0, k16 = -1.0 / 6.0;
+  // ---- forward (weno_sums)
   const P a = psub(u[1], u[0]), b = psub(u[2], u[1]), c = psub(u[3], u[2]), d = psub(u[4], u[3]);
-  const P D2 = psub(b, a), D1 = psub(c, b), D0 = psub(d, c);
-  const P E2 = pfma(b, K(2.0), D2), E1 = padd(b, c), E0 = pfma(c, K(-2.0), D0);
-  const P k313 = K(3.0 / 13.0), eps = K(1e-10 * 12.0 / 13.0);
-  const P B0 = pfma(D0, D0, pfma(pmul(E0, k313), E0, eps));
-  const P B1 = pfma(D1, D1, pfma(pmul(E1, k313), E1, eps));
-  const P B2 = pfma(D2, D2, pfma(pmul(E2, k313), E2, eps));
+  const P t1 = pfma(b, K(-1.25), c), t2 = pfma(b, K(-2.75), a), t0 = pfma(c, K(-2.75), d);
+  const P bb = pfma(b, b, K(eps));
+  const P B1 = pfma(c, t1, bb);
+  const P B2 = pfma(a, t2, pfma(bb, K(2.5), K(-1.5 * eps)));
+  const P B0 = pfma(d, t0, pfma(pmul(c, K(2.5)), c, K(eps)));
+  P r0, r1, r2;
+  rcp3(B0, B1, B2, r0, r1, r2);
   const P diff = psub(B0, B2);
   const P tau = pabs(diff);
-  const P rB0 = prcp(B0), rB1 = prcp(B1), rB2 = prcp(B2);
+  const P z0 = pmul(tau, r0), z1 = pmul(tau, r1), z2 = pmul(tau, r2);  // w_r - 1
   const P one = K(1.0);
-  const P q0 = pfma(tau, rB0, one), q1 = pfma(tau, rB1, one), q2 = pfma(tau, rB2, one);
-  const P t1 = pmul(q1, K(0.6));
-  const P Sm = pfma(q0, K(0.3), pfma(q2, K(0.1), t1));
-  const P Sp = pfma(q0, K(0.1), pfma(q2, K(0.3), t1));
-  const P h1 = pmul(D1, K(0.05));
-  const P em0 = pfma(c, K(0.15), pmul(D0, K(-0.05)));
-  const P ep0 = pfma(c, K(-0.05), pmul(D0, K(1.0 / 30.0)));
-  const P em1 = pfma(E1, K(0.15), h1);
-  const P ep1 = pfma(E1, K(-0.15), h1);
-  const P em2 = pfma(b, K(0.05), pmul(D2, K(1.0 / 30.0)));
-  const P ep2 = pfma(b, K(-0.15), pmul(D2, K(-0.05)));
-  const P Nm = pfma(q2, em2, pfma(q1, em1, pmul(q0, em0)));
-  const P Np = pfma(q2, ep2, pfma(q1, ep1, pmul(q0, ep0)));
-  const P rSm = prcp(Sm), rSp = prcp(Sp);
-  // ---- reverse: vm = q0c + Nm / Sm, vp = q0c + Np / Sp
-  const P tm = pmul(lam_m, rSm), tp = pmul(lam_p, rSp);  // adjoints of Nm, Np
-  const P lSm = pmul(tm, pmul(Nm, rSm)), lSp = pmul(tp, pmul(Np, rSp));  // minus the adjoints of Sm, Sp
-  // adjoints of q_r (with the Sm, Sp signs folded in)
-  const P lq0 = pfma(tp, ep0, pfma(tm, em0, pfma(lSm, K(-0.3), pmul(lSp, K(-0.1)))));
-  const P lq1 = pfma(tp, ep1, pfma(tm, em1, pmul(padd(lSm, lSp), K(-0.6))));
-  const P lq2 = pfma(tp, ep2, pfma(tm, em2, pfma(lSm, K(-0.1), pmul(lSp, K(-0.3)))));
-  // adjoints of the first and second differences through em_r, ep_r (d/d em_r = tm q_r, d/d ep_r = tp q_r)
-  P lc = pmul(q0, pfma(tm, K(0.15), pmul(tp, K(-0.05))));
-  P lD0 = pmul(q0, pfma(tm, K(-0.05), pmul(tp, K(1.0 / 30.0))));
-  P lE1 = pmul(pmul(q1, K(0.15)), psub(tm, tp));
-  P lD1 = pmul(pmul(q1, K(0.05)), padd(tm, tp));
-  P lb = pmul(q2, pfma(tm, K(0.05), pmul(tp, K(-0.15))));
-  P lD2 = pmul(q2, pfma(tm, K(1.0 / 30.0), pmul(tp, K(-0.05))));
-  // q_r = 1 + tau rB_r: d/dtau = rB_r, d/dB_r = -tau rB_r^2 = -(q_r - 1) rB_r
-  const P ltau = pfma(lq2, rB2, pfma(lq1, rB1, pmul(lq0, rB0)));
-  const P sl = pmk(diff.x > R(0) ? ltau.x : (diff.x < R(0) ? -ltau.x : R(0)),
-                   diff.y > R(0) ? ltau.y : (diff.y < R(0) ? -ltau.y : R(0)));
-  // twice the adjoints of B_r (B_r = D_r^2 + 3/13 E_r^2 + eps)
-  const P m2 = K(-2.0);
-  const P lB0 = pfma(pmul(lq0, psub(q0, one)), pmul(rB0, m2), padd(sl, sl));
-  const P lB1 = pmul(pmul(lq1, psub(q1, one)), pmul(rB1, m2));
-  const P lB2 = psub(pmul(pmul(lq2, psub(q2, one)), pmul(rB2, m2)), padd(sl, sl));
-  lD0 = pfma(D0, lB0, lD0);
-  lD1 = pfma(D1, lB1, lD1);
-  lD2 = pfma(D2, lB2, lD2);
-  const P lE0 = pmul(pmul(E0, k313), lB0);
-  lE1 = pfma(pmul(E1, k313), lB1, lE1);
-  const P lE2 = pmul(pmul(E2, k313), lB2);
-  // E2 = 2b + D2, E1 = b + c, E0 = -2c + D0
-  lb = pfma(lE2, K(2.0), padd(lb, lE1));
-  lD2 = padd(lD2, lE2);
-  lc = pfma(lE0, K(-2.0), padd(lc, lE1));
-  lD0 = padd(lD0, lE0);
-  // D2 = b - a, D1 = c - b, D0 = d - c
-  lb = psub(padd(lb, lD2), lD1);
-  lc = psub(padd(lc, lD1), lD0);
-  const P la = pmul(lD2, K(-1.0));
-  const P ld = lD0;
+  const P w0 = padd(z0, one), w1 = padd(z1, one), w2 = padd(z2, one);
+  const P s1 = pmul(w1, K(3.0));
+  const P Sm = pfma(w0, K(1.5), pfma(w2, K(0.5), s1)), Sp = pfma(w0, K(0.5), pfma(w2, K(1.5), s1));
+  const P e0 = pfma(d, K(-0.25), c), e1 = pfma(b, K(0.5), c), e2 = pfma(a, K(k16), pmul(b, K(k512)));
+  const P h0 = pfma(d, K(k16), pmul(c, K(k512))), h1 = pfma(c, K(0.5), b), h2 = pfma(a, K(-0.25), b);
+  const P Nm = pfma(w2, e2, pfma(w1, e1, pmul(w0, e0)));
+  const P Np = pfma(w2, h2, pfma(w1, h1, pmul(w0, h0)));
+  P rm, rp;
+  rcp2(Sm, Sp, rm, rp);
+  // ---- reverse: adjoints tm of Nm, -tp of Np; lm, lp those of Sm, Sp with the opposite sign
+  const P tm = pmul(lam_m, rm), tp = pmul(lam_p, rp);
+  const P lm = pmul(tm, pmul(Nm, rm)), lp = pmul(tp, pmul(Np, rp));
+  // adjoints of w_r (lS = lm - lp enters with the normalisers' weights)
+  const P lw0 = psub(pfma(tm, e0, pmul(lp, K(0.5))), pfma(tp, h0, pmul(lm, K(1.5))));
+  const P lw1 = pfma(psub(lp, lm), K(3.0), psub(pmul(tm, e1), pmul(tp, h1)));
+  const P lw2 = psub(pfma(tm, e2, pmul(lp, K(1.5))), pfma(tp, h2, pmul(lm, K(0.5))));
+  // w_r = 1 + tau r_r: d/dtau = r_r, d/dB_r = -tau r_r^2 = -z_r r_r
+  const P m0 = pmul(lw0, r0), m1 = pmul(lw1, r1), m2 = pmul(lw2, r2);
+  const P lt = padd(padd(m0, m1), m2);
+  const P sl = pmk(diff.x > R(0) ? lt.x : (diff.x < R(0) ? -lt.x : R(0)),
+                   diff.y > R(0) ? lt.y : (diff.y < R(0) ? -lt.y : R(0)));
+  const P lB0 = psub(sl, pmul(m0, z0)), nB1 = pmul(m1, z1), nB2 = pfma(m2, z2, sl);  // dJ/dB0, -dJ/dB1, -dJ/dB2
+  // adjoints of the first differences, through the candidates and through the indicators
+  const P x0 = pmul(tm, w0), x1 = pmul(tm, w1), x2 = pmul(tm, w2);
+  const P y0 = pmul(tp, w0), y1 = pmul(tp, w1), y2 = pmul(tp, w2);
+  P la = pfma(x2, K(k16), pmul(y2, K(0.25)));
+  P lb = psub(pfma(x2, K(k512), pmul(x1, K(0.5))), padd(y1, y2));
+  P lc = psub(padd(x0, x1), pfma(y0, K(k512), pmul(y1, K(0.5))));
+  P ld = pfma(x0, K(-0.25), pmul(y0, K(-k16)));
+  la = psub(la, pmul(nB2, padd(t2, a)));                                       // dB2/da = 2 a - 11/4 b
+  lb = psub(lb, pmul(nB2, pfma(a, K(-2.75), pmul(b, K(5.0)))));                // dB2/db = 5 b - 11/4 a
+  lb = psub(lb, pmul(nB1, pfma(c, K(-1.25), padd(b, b))));                     // dB1/db = 2 b - 5/4 c
+  lc = psub(lc, pmul(nB1, padd(t1, c)));                                       // dB1/dc = 2 c - 5/4 b
+  lc = pfma(lB0, pfma(d, K(-2.75), pmul(c, K(5.0))), lc);                      // dB0/dc = 5 c - 11/4 d
+  ld = pfma(lB0, padd(t0, d), ld);                                             // dB0/dd = 2 d - 11/4 c
   // a = u1 - u0, b = u2 - u1, c = u3 - u2, d = u4 - u3; u2 is also the value both faces start from
   g[0] = psub(g[0], la);
   g[1] = padd(g[1], psub(la, lb));
@@ -173,6 +186,14 @@ __device__ __forceinline__ void adj_g_local(const AdjStageArgs<R>& A, int d, int
   gv += coef * lvel;
 }
 
+// Asynchronous copy of one element into shared memory; zero where !ok (nothing is read then).
+template <class R>
+__device__ __forceinline__ void copy_async(R* dst, const R* src, bool ok) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  const int n = ok ? (int)sizeof(R) : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(sizeof(R)), "r"(n) : "memory");
+}
+
 // Adjoint of one stage kernel launch. CTA = 32 x 16 columns marching up a z chunk, as the forward
 // stage kernel. At centre plane kc: the x and y centres of the tile and its 2-cell halo through
 // shared memory (each centre's five contributions written once, then gathered by the five cells
@@ -220,33 +241,35 @@ __global__ void __launch_bounds__(ANTHREADS, 1) k_adj_stage(const AdjStageArgs<R
     rin[q] = (e < S::TN) && x >= 0 && x < Nx && y >= 0 && y < Ny;
     roff[q] = rin[q] ? (XOFF + x + Sx * (int64_t)y) : 0;
   }
-  R pre[NE][6];
   uint8_t prc[NE];
+  // plane k into raw buffer k & 1, asynchronously (zeros outside the grid); the class bytes, too small
+  // for an asynchronous copy, pass through a register
   auto prefetch = [&](int k) {
-#pragma unroll
-    for (int q = 0; q < NE; q++) {
-      const int64_t g = roff[q] + plane * (int64_t)k;
-      const bool ok = rin[q] && k < Nz && fz_inb(A.err, g, A.nfield);
-      pre[q][0] = ok ? A.pi[g] : R(0);
-      pre[q][1] = ok ? A.ui[g] : R(0);
-      pre[q][2] = ok ? A.vi[g] : R(0);
-      pre[q][3] = ok ? A.lp[g] : R(0);
-      pre[q][4] = ok ? A.lu[g] : R(0);
-      pre[q][5] = ok ? A.lv[g] : R(0);
-      prc[q] = ok ? A.cls[g] : (uint8_t)0;
-    }
-  };
-  auto stash = [&](int buf) {
-    R* raw = sm + buf * S::RAW;
+    R* raw = sm + (k & 1) * S::RAW;
 #pragma unroll
     for (int q = 0; q < NE; q++) {
       const int e = lt + q * ANTHREADS;
-      if (e < S::TN) {
-#pragma unroll
-        for (int f = 0; f < 6; f++) raw[f * S::TN + e] = pre[q][f];
-        clsT[buf * S::TN + e] = prc[q];
-      }
+      if (e >= S::TN) continue;
+      const int64_t g = roff[q] + plane * (int64_t)k;
+      const bool ok = rin[q] && k < Nz && fz_inb(A.err, g, A.nfield);
+      const int64_t at = ok ? g : 0;
+      copy_async(raw + 0 * S::TN + e, A.pi + at, ok);
+      copy_async(raw + 1 * S::TN + e, A.ui + at, ok);
+      copy_async(raw + 2 * S::TN + e, A.vi + at, ok);
+      copy_async(raw + 3 * S::TN + e, A.lp + at, ok);
+      copy_async(raw + 4 * S::TN + e, A.lu + at, ok);
+      copy_async(raw + 5 * S::TN + e, A.lv + at, ok);
+      prc[q] = ok ? A.cls[g] : (uint8_t)0;
     }
+  };
+  // completes the copies of plane k (the caller's barrier publishes them)
+  auto stash = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < NE; q++) {
+      const int e = lt + q * ANTHREADS;
+      if (e < S::TN) clsT[(k & 1) * S::TN + e] = prc[q];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   };
   auto ldz = [&](const R* f, int k) -> R {
     return (col_in && k >= 0 && k < Nz && fz_inb(A.err, col + plane * k, A.nfield)) ? f[col + plane * k] : R(0);
@@ -294,7 +317,7 @@ __global__ void __launch_bounds__(ANTHREADS, 1) k_adj_stage(const AdjStageArgs<R
   R d1p = R(0), d1u = R(0), d1v = R(0), d2p = R(0), d2u = R(0), d2v = R(0);  // x/y sums of kc-1, kc-2
 
   prefetch(kb);
-  stash(kb & 1);
+  stash(kb);
   __syncthreads();  // raw tiles of plane kb stashed
 
   const int nit = (ke - kb) + 4;
@@ -410,7 +433,7 @@ __global__ void __launch_bounds__(ANTHREADS, 1) k_adj_stage(const AdjStageArgs<R
       // second barrier); the barrier below publishes them, so the next plane's weights (the first
       // phase) need no barrier of their own and share a phase with this plane's gather, z centre
       // and flush
-      if (nxt) stash((kc + 1) & 1);
+      if (nxt) stash(kc + 1);
       __syncthreads();
       // cell (i, j) receives offset q - 2 of the x centre i - (q - 2) and of the y centre j - (q - 2)
 #pragma unroll
@@ -521,14 +544,7 @@ __global__ void __launch_bounds__(256) k_adj_band(const AdjBandArgs<R> B) {
   const R nx = B.nrm[4 * b + 0], ny = B.nrm[4 * b + 1], nz = B.nrm[4 * b + 2];
   const int64_t Sx = B.Sx, pl = B.plane;
   // forward values needed by the linearisation (the probe as the forward evaluates it)
-  auto tri = [&](const R* f) {
-    const R c00 = f[q] * (R(1) - sx) + f[q + 1] * sx;
-    const R c10 = f[q + Sx] * (R(1) - sx) + f[q + Sx + 1] * sx;
-    const R c01 = f[q + pl] * (R(1) - sx) + f[q + pl + 1] * sx;
-    const R c11 = f[q + pl + Sx] * (R(1) - sx) + f[q + pl + Sx + 1] * sx;
-    const R c0 = c00 * (R(1) - sy) + c10 * sy, c1 = c01 * (R(1) - sy) + c11 * sy;
-    return c0 * (R(1) - sz) + c1 * sz;
-  };
+  auto tri = [&](const R* f) { return trilin<R>(f, q, Sx, pl, sx, sy, sz); };
   const R pD = tri(B.pi), uD = tri(B.ui), vD = tri(B.vi), wD = tri(B.wi);
   const R un = uD * nx + vD * ny + wD * nz;
   const double Z0 = B.Z0, dt = B.dt;
@@ -619,6 +635,7 @@ __global__ void __launch_bounds__(256) k_adj_probe_scatter(const AdjBandArgs<R> 
                    (R(1) - sx) * sy * sz,                    sx * sy * sz};
 #pragma unroll
   for (int e = 0; e < 8; e++) {
+    if (wt[e] == R(0)) continue;  // a probe on a cell plane (walls along the grid) has fewer corners
     const int64_t x = q + off[e];
     atomicAdd(B.ip + x, wt[e] * lpD);
     atomicAdd(B.iu + x, wt[e] * luD);
