@@ -718,9 +718,9 @@ __global__ void __launch_bounds__(256) k_adj_pml_grad(const AdjPmlArgs<R> A) {
 #pragma unroll
     for (int o = 0; o < 7; o++) q[o] = pmk(A.pi[g + (o - 3) * st], A.vi[g + (o - 3) * st]);
     P ml, pl, mc, pc, mr, pr;
-    weno_center<R>(q[0], q[1], q[2], q[3], q[4], ml, pl);
-    weno_center<R>(q[1], q[2], q[3], q[4], q[5], mc, pc);
-    weno_center<R>(q[2], q[3], q[4], q[5], q[6], mr, pr);
+    weno_center(q[0], q[1], q[2], q[3], q[4], ml, pl);
+    weno_center(q[1], q[2], q[3], q[4], q[5], mc, pc);
+    weno_center(q[2], q[3], q[4], q[5], q[6], mr, pr);
     const P L = psub(godunov<R>(ml, pc, kA, kC), godunov<R>(mc, pr, kA, kC));
     const R Dp = L.x * A.inv_h, Dv = L.y * A.inv_h;
     atomicAdd(&gs[3 * tile], A.wdt * ((double)A.lp[g] * (double)Dp + (double)A.lv[g] * (double)Dv));

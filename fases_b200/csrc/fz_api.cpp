@@ -557,14 +557,26 @@ fz::StageArgs<R> stage_args(fz_handle* h, int stage) {
   for (int c = 0; c < h->zchunks && c < fz::FZ_MAX_ZCHUNKS; c++) a.zoff[c + 1] = a.zoff[c] + h->zsizes[(size_t)c];
   const fz_params& p = h->prm;
   a.z0 = (R)(p.rho * p.c);
-  a.dt_p = (R)(0.5 * p.dt * p.c / p.h);
-  a.dt_v = (R)(0.5 * p.dt / (p.h * p.rho));
-  a.ih_p = (R)(0.5 * p.c / p.h);
-  a.ih_v = (R)(0.5 / (p.h * p.rho));
+  a.frc2 = (R)(0.5 * p.rho * p.c * p.c);
+  a.firho = (R)(0.5 / p.rho);
+  a.fc = (R)(0.5 * p.c);
+  const bool waves = sizeof(R) == 8;
+  a.dt_p = (R)(waves ? 0.5 * p.dt * p.c / p.h : p.dt / p.h);
+  a.dt_v = (R)(waves ? 0.5 * p.dt / (p.h * p.rho) : p.dt / p.h);
+  a.ih_p = (R)(waves ? 0.5 * p.c / p.h : 1.0 / p.h);
+  a.ih_v = (R)(waves ? 0.5 / (p.h * p.rho) : 1.0 / p.h);
   const double w = (stage == 0) ? 1.0 : (stage == 1) ? 0.25 : 2.0 / 3.0;
   a.wdt = (R)(w * p.dt);
   a.pml_on = h->pml_on ? 1 : 0;
   a.pml_d2 = 2 * p.pml_cells;
+  {
+    const int n[3] = {h->Nx, h->Ny, h->Nz};
+    const int lo[3] = {p.pml[3], p.pml[5], p.pml[1]}, hi[3] = {p.pml[2], p.pml[4], p.pml[0]};
+    for (int q = 0; q < 3; q++) {
+      a.pml_lo[q] = lo[q] ? GHOST + p.pml_cells : 0;
+      a.pml_hi[q] = hi[q] ? n[q] - GHOST - p.pml_cells : n[q];
+    }
+  }
   a.pcx = (const fz::PmlCoef<R>*)h->d_pml_coef[0];
   a.pcy = (const fz::PmlCoef<R>*)h->d_pml_coef[1];
   a.pcz = (const fz::PmlCoef<R>*)h->d_pml_coef[2];
@@ -580,7 +592,15 @@ fz::StageArgs<R> stage_args(fz_handle* h, int stage) {
   a.src_opt = h->src_opt;
   a.src_w = (R)w;
   a.nn_mul = 2;
-  a.nn_add = (stage == 0) ? 0 : (stage == 1) ? 2 : 1;  // main3D.cu:1288, 1296, 1304
+  a.nn_add = ((stage == 0) ? 0 : (stage == 1) ? 2 : 1) + 2 * h->seq;  // main3D.cu:1288, 1296, 1304
+  if (stage == 0 && h->seq > 0) {  // the previous step of this run, recorded from this stage's input
+    a.rec_n = h->nrec * h->nb;
+    a.rec_off = h->seq - 1;
+    a.rcell = h->d_rec_cell;
+    a.ir = h->d_ir;
+    a.vel = h->d_vel;
+    a.rec_cap = h->rec_cap;
+  }
   a.half_dt = (R)(0.5 * p.dt);
   a.step = h->d_step;
   a.err = h->d_err;
@@ -706,8 +726,9 @@ cudaError_t enqueue_finish(fz_handle* h) {
     Timer t(h, 4);
     R* const* u1 = (R* const*)h->U[h->i1];
     e = fz::launch_receivers<R>(u1[0], u1[1], u1[2], u1[3], h->d_rec_cell, h->nrec * h->nb, h->d_ir, h->d_vel,
-                                h->rec_cap, h->d_step, h->d_err, h->ncell_dev * h->nb, h->stream);
+                                h->rec_cap, h->d_step, h->seq, h->d_err, h->ncell_dev * h->nb, h->stream);
     if (e != cudaSuccess) return e;
+    h->seq = 0;
     if (h->sl_on) {
       e = fz::launch_slices<R>(u1[0], u1[1], u1[2], u1[3], h->Nx, h->Ny, h->Nz, h->Sx, h->sl_i, h->sl_j, h->sl_k,
                                h->d_step, h->sl_step, h->sl_cap, h->d_slices, h->nsm, h->stream);
@@ -729,6 +750,26 @@ cudaError_t enqueue_step(fz_handle* h) {
   return enqueue_finish<R>(h);
 }
 
+// n steps in a row: the samples of each but the last are recorded by the stage 0 launch that follows,
+// which saves their launch from the chain of dependent ones. Animation frames and per-kernel timings
+// are taken after every step.
+template <class R>
+cudaError_t enqueue_steps(fz_handle* h, int n) {
+  cudaError_t e = cudaSuccess;
+  const bool every = h->sl_on || h->profiling;
+  for (int s = 0; s < n && e == cudaSuccess; s++) {
+    if (every || s + 1 == n) {
+      e = enqueue_step<R>(h);
+      continue;
+    }
+    for (int st = 0; st < 3 && e == cudaSuccess; st++) e = enqueue_stage<R>(h, st);
+    fzi::rotate(h);
+    h->seq++;
+  }
+  if (e != cudaSuccess) h->seq = 0;
+  return e;
+}
+
 // Captures and instantiates the graph of G steps for the current buffer parity (h->i0), unless it
 // exists. Capture advances the host-side rotation by G (even) steps: back where it started.
 template <class R>
@@ -738,8 +779,7 @@ int ensure_graph(fz_handle* h) {
   if (h->graph[par]) return FZ_OK;
   cudaGraph_t g = nullptr;
   FZ_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-  cudaError_t e = cudaSuccess;
-  for (int s = 0; s < G && e == cudaSuccess; s++) e = enqueue_step<R>(h);
+  cudaError_t e = enqueue_steps<R>(h, G);
   cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
   if (e != cudaSuccess) return cuda_fail(h, e, "capture step");
   if (e2 != cudaSuccess) return cuda_fail(h, e2, "end capture");
@@ -790,10 +830,12 @@ int run_steps(fz_handle* h, int64_t nsteps) {
       h->steps_enqueued += G;
     }
   }
-  for (; done < nsteps; done++) {
-    cudaError_t e = enqueue_step<R>(h);
+  while (done < nsteps) {
+    const int n = (int)std::min<int64_t>(nsteps - done, 16);
+    cudaError_t e = enqueue_steps<R>(h, n);
     if (e != cudaSuccess) return cuda_fail(h, e, "step launch");
-    h->steps_enqueued += 1;
+    h->steps_enqueued += n;
+    done += n;
   }
   return FZ_OK;
 }

@@ -30,9 +30,38 @@ __device__ __forceinline__ R source_sum(const StageArgs<R>& A, int64_t g) {
   return add;
 }
 
+// Receiver samples of a completed step (main3D.cu:1399-1414) into trace column n, by the threads
+// t = 0 .. nt-1; a non-finite sample sets the health word.
+template <class R>
+__device__ __forceinline__ void record_samples(const R* p, const R* u, const R* v, const R* w, const int64_t* rcell,
+                                               int nrec, double* ir, double* vel, int64_t cap, int64_t n,
+                                               int32_t* err, int64_t nfield, int t, int nt) {
+  for (int r = t; r < nrec; r += nt) {
+    const int64_t c = rcell[r];
+    if (!fz_inb(err, c, nfield)) continue;
+    const double pp = (double)p[c], uu = (double)u[c], vv = (double)v[c], ww = (double)w[c];
+    // health word: a blown-up solution reaches the receivers (their samples are read anyway)
+    if (!isfinite(pp) || !isfinite(uu) || !isfinite(vv) || !isfinite(ww)) atomicOr(err, KERR_NONFINITE);
+    if (n < cap) {
+      const int64_t o = (int64_t)r * cap + n;
+      ir[o] = pp;
+      vel[3 * o + 0] = uu;
+      vel[3 * o + 1] = vv;
+      vel[3 * o + 2] = ww;
+    }
+  }
+}
+// The previous step's samples, by the threads of one block of a stage 0 launch: the step's result is
+// the stage's input, so this needs no launch of its own between the steps.
+template <class R>
+__device__ __noinline__ void stage_receivers(const StageArgs<R>& A, int t, int nt) {
+  record_samples<R>(A.pi, A.ui, A.vi, A.wi, A.rcell, A.rec_n, A.ir, A.vel, A.rec_cap, *A.step + A.rec_off, A.err,
+                    A.nfield, t, nt);
+}
+
 // cPML (functions3D.cuh:725-755): field += w dt ((1/kappa - 1) D + psi), psi frozen within the step
-// and advanced once, in stage 2, by recursive convolution. D*: (X - Y, X + Y) of the
-// characteristics' differences along each axis; cx, cy, cz: the cell's coefficients.
+// and advanced once, in stage 2, by recursive convolution. D*: the differences
+// along each axis as Sweep gives them; cx, cy, cz: the cell's coefficients.
 template <class R, int STAGE>
 __device__ __forceinline__ void pml_axis(const StageArgs<R>& A, typename Pair<R>::T* psi, int64_t at,
                                          const PmlCoef<R>& c, typename Pair<R>::T D, R& p, R& vel) {
@@ -71,12 +100,12 @@ template <class R>
 __device__ __forceinline__ R trilin(const R* __restrict__ f, int64_t q, int64_t Sx, int64_t plane, R sx,
                                     R sy, R sz) {
   const R ox = R(1) - sx, oy = R(1) - sy, oz = R(1) - sz;
-  const R c00 = fma(__ldg(f + q + 1), sx, __ldg(f + q) * ox);
-  const R c10 = fma(__ldg(f + q + Sx + 1), sx, __ldg(f + q + Sx) * ox);
-  const R c01 = fma(__ldg(f + q + plane + 1), sx, __ldg(f + q + plane) * ox);
-  const R c11 = fma(__ldg(f + q + plane + Sx + 1), sx, __ldg(f + q + plane + Sx) * ox);
-  const R c0 = fma(c10, sy, c00 * oy), c1 = fma(c11, sy, c01 * oy);
-  return fma(c1, sz, c0 * oz);
+  const R c00 = fma(__ldg(f + q), ox, __ldg(f + q + 1) * sx);
+  const R c10 = fma(__ldg(f + q + Sx), ox, __ldg(f + q + Sx + 1) * sx);
+  const R c01 = fma(__ldg(f + q + plane), ox, __ldg(f + q + plane + 1) * sx);
+  const R c11 = fma(__ldg(f + q + plane + Sx), ox, __ldg(f + q + plane + Sx + 1) * sx);
+  const R c0 = fma(c00, oy, c10 * sy), c1 = fma(c01, oy, c11 * sy);
+  return fma(c0, oz, c1 * sz);
 }
 
 template <class R>
@@ -128,7 +157,7 @@ __device__ __forceinline__ void ade_pair(double& r1, double& r2, double m1, doub
 // With K = L = 2 a band cell moves 176 instead of 384 bytes of states a step, with the same bits.
 // KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
 // probe is then issued at the top, beside the probe gathers, so one thread keeps ~50 loads in flight;
-// KM = LM = 0 is the general form with the state loads inside the pole loops.
+// KM = LM = 0 is the general form with the state loads inside the pole loops; it keeps every state.
 template <class R, int STAGE, int KM, int LM, bool KEEP>
 __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b, const int64_t cell, const int4& rc,
                                           R& p, R& u, R& v, R& w) {
@@ -158,18 +187,18 @@ __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b,
       }
     }
   double w0 = 0.0, w1 = 0.0;  // the outgoing characteristics of the earlier stages
-  if (!KEEP && STAGE > 0) w0 = __ldg(B.wst + b);
-  if (!KEEP && STAGE > 1) w1 = __ldg(B.wst + nB + b);
+  if (KM > 0 && !KEEP && STAGE > 0) w0 = __ldg(B.wst + b);
+  if (KM > 0 && !KEEP && STAGE > 1) w1 = __ldg(B.wst + nB + b);
   const R sx = g4.x, sy = g4.y, sz = g4.z, chi = g4.w;
   const R nx = n4.x, ny = n4.y, nz = n4.z;
   const R pD = trilin<R>(B.pi, q, B.Sx, B.plane, sx, sy, sz);
   const R uD = trilin<R>(B.ui, q, B.Sx, B.plane, sx, sy, sz);
   const R vD = trilin<R>(B.vi, q, B.Sx, B.plane, sx, sy, sz);
   const R wD = trilin<R>(B.wi, q, B.Sx, B.plane, sx, sy, sz);
-  const R un = fma(wD, nz, fma(vD, ny, uD * nx));
+  const R un = fma(wD, nz, fma(uD, nx, vD * ny));
   const R utx = fma(-un, nx, uD), uty = fma(-un, ny, vD), utz = fma(-un, nz, wD);
   const double wout = fma(B.Z0, (double)un, (double)pD);  // outgoing characteristic
-  if (!KEEP && STAGE < 2) B.wst[STAGE * nB + b] = wout;
+  if (KM > 0 && !KEEP && STAGE < 2) B.wst[STAGE * nB + b] = wout;
   const double dt = B.dt;
   double sumA = 0.0, sumBC = 0.0;
   auto real_pole = [&](int k, double r, double mid) {
@@ -197,7 +226,7 @@ __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b,
       B.s1L[si] = r1;
       B.s2L[si] = r2;
     }
-    sumBC = fma(__ldg(B.B + mi), r1, fma(__ldg(B.C + mi), r2, sumBC));
+    sumBC += fma(__ldg(B.B + mi), r1, __ldg(B.C + mi) * r2);
   };
   if constexpr (KM > 0) {
 #pragma unroll
@@ -206,24 +235,62 @@ __device__ __forceinline__ void band_cell(const BandArgs<R>& B, const int64_t b,
 #pragma unroll
     for (int l = 0; l < LM; ++l)
       if (l < B.L) pole_pair(l, r1L[l], r2L[l], m1L[l], m2L[l]);
+  }
+  double win;  // incoming characteristic
+  if constexpr (KM > 0) {
+    win = fma(__ldg(B.Rinf + m), wout, sumA) + sumBC;
   } else {
+    // any number of poles: the states after every stage are kept, the products left to the compiler to
+    // contract, as this form has always been built
+    constexpr double a_ssp = (STAGE == 0) ? 0.0 : (STAGE == 1) ? 3.0 : 1.0;
+    constexpr double b_ssp = (STAGE == 2) ? 2.0 : 1.0;
+    constexpr double inv_c = (STAGE == 0) ? 1.0 : (STAGE == 1) ? 0.25 : 1.0 / 3.0;
+    auto real = [&](int k, double r, double mid) {
+      const int mi = m * B.K + k;
+      const double Lphi = wout - __ldg(B.zeta + mi) * r;
+      double v = b_ssp * (r + B.dt * Lphi);
+      if (STAGE > 0) v += a_ssp * mid;
+      v *= inv_c;
+      B.phL[(int64_t)k * nB + b] = v;
+      sumA += __ldg(B.A + mi) * v;
+    };
+    auto pair = [&](int l, double r1, double r2, double m1, double m2) {
+      const int mi = m * B.L + l;
+      const double al = __ldg(B.alpha + mi), be = __ldg(B.beta + mi);
+      const double L1 = wout - (al * r1 + be * r2);
+      const double L2 = be * r1 - al * r2;
+      double n1 = b_ssp * (r1 + B.dt * L1);
+      double n2 = b_ssp * (r2 + B.dt * L2);
+      if (STAGE > 0) {
+        n1 += a_ssp * m1;
+        n2 += a_ssp * m2;
+      }
+      n1 *= inv_c;
+      n2 *= inv_c;
+      const int64_t si = (int64_t)l * nB + b;
+      B.s1L[si] = n1;
+      B.s2L[si] = n2;
+      sumBC += __ldg(B.B + mi) * n1 + __ldg(B.C + mi) * n2;
+    };
     for (int k = 0; k < B.K; ++k) {
       const int64_t si = (int64_t)k * nB + b;
-      real_pole(k, RIGHT ? B.phR[si] : 0.0, B.phM[si]);
+      real(k, B.phR[si], STAGE > 0 ? B.phM[si] : 0.0);
     }
     for (int l = 0; l < B.L; ++l) {
       const int64_t si = (int64_t)l * nB + b;
-      pole_pair(l, RIGHT ? B.s1R[si] : 0.0, RIGHT ? B.s2R[si] : 0.0, B.s1M[si], B.s2M[si]);
+      pair(l, B.s1R[si], B.s2R[si], STAGE > 0 ? B.s1M[si] : 0.0, STAGE > 0 ? B.s2M[si] : 0.0);
     }
+    win = __ldg(B.Rinf + m) * wout + sumA + sumBC;
   }
-  const double win = fma(__ldg(B.Rinf + m), wout, sumA + sumBC);  // incoming characteristic
   const R pb = (R)(0.5 * (win + wout));
   const R unb = (R)((wout - win) / (2.0 * B.Z0));
   const R omc = R(1) - chi;
-  u = fma(chi, fma(unb, nx, utx), omc * u);
-  v = fma(chi, fma(unb, ny, uty), omc * v);
-  w = fma(chi, fma(unb, nz, utz), omc * w);
-  p = fma(chi, pb, omc * p);
+  u = fma(omc, u, chi * fma(unb, nx, utx));
+  v = fma(omc, v, chi * fma(unb, ny, uty));
+  // (which product is the rounded one differs between the forms, as they have always been contracted)
+  const R wb = fma(unb, nz, utz);
+  w = KM > 0 ? fma(omc, w, chi * wb) : fma(chi, wb, omc * w);
+  p = fma(omc, p, chi * pb);
 }
 
 }  // namespace fz

@@ -86,14 +86,17 @@ struct StageArgs {
   // chunk c of a member covers its interior planes [zoff[c], zoff[c+1]) (counted from the first
   // interior plane); chunks may differ in length (long ones first, short ones for the last waves)
   int32_t zoff[FZ_MAX_ZCHUNKS + 1];
+  // flux constants (Sweep in fz_pair.cuh): FP32 dt_p = dt_v = dt / h of flux differences; FP64 dt c / 2h and
+  // dt / 2 rho h of the characteristics' differences and sums; ih_p, ih_v the same without dt (cPML)
+  R dt_p, dt_v, ih_p, ih_v;
   R z0;     // rho * c
-  R dt_p;   // dt / h * c / 2: p per difference of the characteristics
-  R dt_v;   // dt / h / (2 rho): velocity per sum of the characteristics
-  R ih_p;   // 1 / h * c / 2 (the cPML's flux differences)
-  R ih_v;   // 1 / h / (2 rho)
+  R frc2;   // 0.5 * rho * c^2
+  R firho;  // 0.5 / rho
+  R fc;     // 0.5 * c
   R wdt;    // stage weight * dt (cPML correction weight)
-  // cPML (pml_on = 0: no face enabled)
+  // cPML (pml_on = 0: no face enabled); cells of a layer: index < pml_lo or >= pml_hi along the axis
   int32_t pml_on;
+  int32_t pml_lo[3], pml_hi[3];
   int32_t pml_d2;  // 2 * pml_cells
   const PmlCoef<R>* pcx;
   const PmlCoef<R>* pcy;
@@ -114,6 +117,14 @@ struct StageArgs {
   R half_dt;
   const int64_t* step;  // device step counter n
   int32_t* err;         // set to a nonzero FZ_KERR_* code when a bounded wait gives up
+  // stage 0 of a step that follows another in the same run: the receiver samples of that step (its
+  // result is this stage's input), sample *step + rec_off; rec_n = 0 otherwise
+  int32_t rec_n;
+  int32_t rec_off;
+  const int64_t* rcell;
+  double* ir;
+  double* vel;
+  int64_t rec_cap;
   // array sizes for the bounds-checked build: elements of one field array (all members), of the
   // psi tiles per axis, of the cPML tables per axis
   int64_t nfield;

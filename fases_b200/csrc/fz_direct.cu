@@ -35,12 +35,16 @@ template <class R, int STAGE, bool DIM2, int KM, int LM>
 __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArgs<R>& B, const DirectArgs& D, int bx,
                                             int by, int bz) {
   typedef typename Pair<R>::T P;
+  typedef Sweep<R> Sw;
+  typedef typename Sw::X X;
   const int lane = threadIdx.x;
   const int i = GHOST - 1 + bx * DCELLS + lane;
   const int il = min(i, A.Nx - GHOST);  // lanes past the room's end load its last halo centre's column
   const int member = bz / D.chunks, chunk = bz - member * D.chunks;
   const int kz = member * A.Nz;  // this member's first plane
   int j, m0, m1;                 // row (3D), march range
+  if (STAGE == 0 && A.rec_n > 0 && bx == 0 && by == 0 && bz == 0)
+    stage_receivers<R>(A, (int)threadIdx.y * 32 + lane, 32 * DROWS);
   if (!DIM2) {
     j = GHOST + by * DROWS + threadIdx.y;
     m0 = GHOST + chunk * D.depth;
@@ -62,13 +66,17 @@ __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArg
 
   // march queue: centres m0-1 and m0, then one centre ahead per cell
   P qa, qb, qc, qd;
-  R zr_lo, zr, zl;
+  X mlo, m_below, mhi;  // lo of centre m; planar rooms: lo of m - 1 and hi of m as well
+  typename Sw::F Fm_lo;
   {
     const P z0 = ldq(g - 3 * ms), z1 = ldq(g - 2 * ms), z2 = ldq(g - ms), z3 = ldq(g), z4 = ldq(g + ms);
     const P z5 = ldq(g + 2 * ms);
-    R unused;
-    weno_waves<R, WENO_LO>(z0, z1, z2, z3, z4, A.z0, zr_lo, unused);
-    weno_waves<R>(z1, z2, z3, z4, z5, A.z0, zr, zl);
+    X lo, hi, unused;
+    Sw::template centre<WENO_LO>(A, z0, z1, z2, z3, z4, lo, unused);
+    Sw::centre(A, z1, z2, z3, z4, z5, mlo, hi);
+    Fm_lo = Sw::face(A, lo, hi);
+    m_below = lo;
+    mhi = hi;
     qa = z2; qb = z3; qc = z4; qd = z5;
   }
   for (int m = m0; m < m1; ++m, g += ms) {
@@ -100,27 +108,34 @@ __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArg
     if (KM >= 0 && b >= 0) rc = __ldg(B.rec + b);
 
     // ---- centres
-    R zr_hi, zl_hi, xr, xl;
-    weno_waves<R>(qa, qb, qc, qd, qe, A.z0, zr_hi, zl_hi);
-    weno_waves<R>(x[0], x[1], x[2], x[3], x[4], A.z0, xr, xl);
-    const R xr_lo = __shfl_up_sync(FULL, xr, 1), xl_hi = __shfl_down_sync(FULL, xl, 1);
-    R yr_lo = R(0), yr = R(0), yl = R(0), yl_hi = R(0);
+    X mlo_up, mhi_up, xlo, xhi;
+    Sw::centre(A, qa, qb, qc, qd, qe, mlo_up, mhi_up);
+    const typename Sw::F Fm_hi = Sw::face(A, mlo, mhi_up);
+    Sw::centre(A, x[0], x[1], x[2], x[3], x[4], xlo, xhi);
+    const X xlo_below = shfl_up1(xlo), xhi_above = shfl_down1(xhi);
+    X ylo_below, ylo, yhi, yhi_above;
     if (!DIM2) {
-      R unused;
-      weno_waves<R, WENO_LO>(y[0], y[1], y[2], y[3], y[4], A.z0, yr_lo, unused);
-      weno_waves<R>(y[1], y[2], y[3], y[4], y[5], A.z0, yr, yl);
-      weno_waves<R, WENO_HI>(y[2], y[3], y[4], y[5], y[6], A.z0, unused, yl_hi);
+      X unused;
+      Sw::template centre<WENO_LO>(A, y[0], y[1], y[2], y[3], y[4], ylo_below, unused);
+      Sw::centre(A, y[1], y[2], y[3], y[4], y[5], ylo, yhi);
+      Sw::template centre<WENO_HI>(A, y[2], y[3], y[4], y[5], y[6], unused, yhi_above);
     }
 
     // ---- the cell's update, as in the marching kernel: stage combination, cPML, sources, band
     if (cls & (CLS_UPDATE | CLS_SOURCE | CLS_BAND)) {
       R pn, un, vn, wn;
       if (cls & CLS_UPDATE) {
-        const R Xx = xr_lo - xr, Yx = xl - xl_hi;
-        const R Xm = zr_lo - zr, Ym = zl - zl_hi;
-        const R Xy = DIM2 ? Xm : yr_lo - yr, Yy = DIM2 ? Ym : yl - yl_hi;
-        const R Xz = DIM2 ? R(0) : Xm, Yz = DIM2 ? R(0) : Ym;
-        const P Dx = pmk(Xx - Yx, Xx + Yx), Dy = pmk(Xy - Yy, Xy + Yy), Dz = pmk(Xz - Yz, Xz + Yz);
+        const P Dx = Sw::across(A, xlo_below, xhi, xlo, xhi_above);
+        // a planar room's march is its y sweep; the marching kernel takes y differences from the states
+        const P Dm = DIM2 ? P() : Sw::across(Fm_lo, Fm_hi);
+        P Dy, Dz;
+        if (DIM2) {
+          Dy = Sw::across(A, m_below, mhi, mlo, mhi_up);
+          Dz = pmk(R(0), R(0));
+        } else {
+          Dy = Sw::across(A, ylo_below, yhi, ylo, yhi_above);
+          Dz = Dm;
+        }
         pn = fma(A.dt_p, (Dx.x + Dy.x) + Dz.x, qb.x);
         un = fma(A.dt_v, Dx.y, x[2].y);
         vn = fma(A.dt_v, Dy.y, v_in);
@@ -132,7 +147,10 @@ __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArg
           vn = fma(wb, vn - bv, bv);
           wn = fma(wb, wn - bw, bw);
         }
-        if (A.pml_on && fz_inb(A.err, k, A.npc[2])) {
+        // layers by index: no coefficient is read where there is none
+        const int kl = DIM2 ? GHOST : m;
+        if (A.pml_on && (i < A.pml_lo[0] || i >= A.pml_hi[0] || jj < A.pml_lo[1] || jj >= A.pml_hi[1] ||
+                         kl < A.pml_lo[2] || kl >= A.pml_hi[2]) && fz_inb(A.err, k, A.npc[2])) {
           const PmlCoef<R> cx = A.pcx[i], cy = A.pcy[jj], cz = A.pcz[k];
           pml_update<R, STAGE>(A, i, jj, k, cx, cy, cz, Dx, Dy, Dz, pn, un, vn, wn);
         }
@@ -156,9 +174,12 @@ __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArg
         A.wo[g] = wn;
       }
     }
-    zr_lo = zr;
-    zr = zr_hi;
-    zl = zl_hi;
+    Fm_lo = Fm_hi;
+    if (DIM2) {
+      m_below = mlo;
+      mhi = mhi_up;
+    }
+    mlo = mlo_up;
     qa = qb;
     qb = qc;
     qc = qd;

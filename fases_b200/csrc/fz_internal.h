@@ -113,6 +113,9 @@ struct fz_handle {
   int64_t* d_step = nullptr;
   double* d_scratch = nullptr;
   int64_t steps_enqueued = 0;
+  // steps enqueued since the device step counter's value: a run of several steps advances the counter
+  // once, and records the samples of all but its last step in the stage 0 launch that follows
+  int seq = 0;
   bool finalized = false;
   int kz_chunk = 0;       // largest z chunk of the stage kernels
   int kz_heuristic = 0;  // the wave-filling choice of prepare (fz_set_kz_chunk(h, 0) returns to it)

@@ -90,9 +90,12 @@ struct StageSmem {
   static constexpr int CLSB = ((TX * TY + 127) / 128) * 128;                     // class bytes
   static constexpr int BUF = 3 * FIELD + 4 * OWN + CLSB;         // p,u,v halo | U0 own | cls
   static constexpr int TILES = NBUF * BUF;
-  static constexpr int XC = TY * (TX + 2);                         // one characteristic of the x-centres
-  static constexpr int YC = (TY + 2) * TX;                         // one characteristic of the y-centres
-  static constexpr int CENTRES = 2 * (2 * XC + 2 * YC) * (int)sizeof(R);  // double buffered (wr, wl) x and y
+  typedef typename Sweep<R>::X X;
+  // one row pitch for both, so that a thread addresses every array from one register
+  static constexpr int CP = TX + 2;
+  static constexpr int XC = TY * CP;        // one array of the x-centres (lo or hi)
+  static constexpr int YC = (TY + 2) * CP;  // one array of the y-centres
+  static constexpr int CENTRES = 2 * (2 * XC + 2 * YC) * (int)sizeof(X);  // double buffered (lo, hi) x and y
   static constexpr int BYTES = TILES + CENTRES + 64 + 128;         // + mbarriers + base alignment
 };
 
@@ -117,6 +120,7 @@ struct StageSmem {
 // DIM2: planar solve (one updated z-plane, no z fluxes): the 3D scheme restricted to 2D.
 // CTA coordinates of a stage-kernel launch of one room: the launch grid itself.
 struct GridCta {
+  static constexpr int planes = 2;  // planes per iteration of the FP32 stage loop
   static __device__ __forceinline__ int x() { return blockIdx.x; }
   static __device__ __forceinline__ int y() { return blockIdx.y; }
   static __device__ __forceinline__ int z() { return blockIdx.z; }
@@ -127,6 +131,8 @@ struct GridCta {
 template <class R, int STAGE, bool DIM2, class CTA>
 __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMaps& M) {
   typedef typename Pair<R>::T P;
+  typedef Sweep<R> Sw;
+  typedef typename Sw::X X;
   typedef StageSmem<R> L;
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   // TMA destinations must be 128-byte aligned: align the base explicitly
@@ -159,6 +165,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
   const int ke = min(GHOST + member * A.Nz + A.zoff[chunk + 1], (member + 1) * A.Nz - GHOST);
   if (kb >= ke) return;
   const int nplanes = ke - kb;
+  if (STAGE == 0 && A.rec_n > 0 && CTA::x() == 0 && CTA::y() == 0 && CTA::z() == 0) stage_receivers<R>(A, lt, NTHREADS);
   const int64_t Sx = A.Sx, plane = A.plane;
   const bool col_ok = (j < A.Ny) && (XOFF + i < Sx);
   const int64_t col = XOFF + i + Sx * (int64_t)j;
@@ -218,17 +225,19 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
     return pmk(A.pi[g], A.wi[g]);
   };
 
-  // z prologue: centres kb-1 and kb give the characteristics at face kb-1/2 and wr at kb+1/2.
+  // z prologue: centres kb-1 and kb give the face kb-1/2 and the lo of face kb+1/2.
   const P zero = psplat<R>(R(0));
   P qa = zero, qb = zero, qc = zero, qd = zero, qe_next = zero;
-  R zr_lo = R(0), zr = R(0), zl = R(0);  // wr(k-1), wr(k), wl(k)
+  X zlo = X();
+  typename Sw::F Fz_lo = typename Sw::F();
   if (!DIM2) {
     const P z0 = ld_pw(kb - 3), z1 = ld_pw(kb - 2), z2 = ld_pw(kb - 1), z3 = ld_pw(kb), z4 = ld_pw(kb + 1);
     const P z5 = ld_pw(kb + 2);
     qe_next = ld_pw(kb + 3);
-    R unused;
-    weno_waves<R, WENO_LO>(z0, z1, z2, z3, z4, A.z0, zr_lo, unused);
-    weno_waves<R>(z1, z2, z3, z4, z5, A.z0, zr, zl);
+    X lo, hi, unused;
+    Sw::template centre<WENO_LO>(A, z0, z1, z2, z3, z4, lo, unused);
+    Sw::centre(A, z1, z2, z3, z4, z5, zlo, hi);
+    Fz_lo = Sw::face(A, lo, hi);
     // queue of plane values k-1 .. k+2 for the centre of plane k+1
     qa = z2; qb = z3; qc = z4; qd = z5;
   }
@@ -241,22 +250,32 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
   const bool pml_zc = A.pml_on && fz_inb(A.err, ke - 1, A.npc[2]) && (A.pcz[kb].tile >= 0 || A.pcz[ke - 1].tile >= 0);
   int buf = 0;
   uint32_t parity = 0;
-  int64_t gk = col + plane * kb;  // offset of (i, j, k)
-  int64_t gz = colz + plane * (kb + 4);  // z-queue load of the next iteration (plane k + 4)
-  for (int it = 0; it < nplanes; ++it, gk += plane, gz += plane) {
+  // 32-bit offsets: 12 field arrays of 2^32 elements do not fit the device
+  const uint32_t plane32 = (uint32_t)plane;
+  uint32_t gk = (uint32_t)(col + plane * kb);          // offset of (i, j, k)
+  uint32_t gz = (uint32_t)(colz + plane * (kb + 4));  // z-queue load of the next iteration (plane k + 4)
+  // two planes an iteration (FP32): the queue's moves between planes and the buffer parity fall away
+  // (500 x 400 x 200, with the 32-bit offsets and the common row pitch above: a stage 0.685 / 0.716 /
+  // 0.718 ms, one plane an iteration 0.708 / 0.728 / 0.731; three 0.719 / 0.778 / 0.782, four 0.707 /
+  // 0.737 / 0.741, both spilling)
+#pragma unroll (sizeof(R) == 4 && !DIM2 ? CTA::planes : 1)
+  for (int it = 0; it < nplanes; ++it, gk += plane32, gz += plane32) {
     const int k = kb + it;
-    R* XR = reinterpret_cast<R*>(cbase) + (it & 1) * (2 * L::XC + 2 * L::YC);
-    R* XL = XR + L::XC;
-    R* YR = XL + L::XC;
-    R* YL = YR + L::YC;
+    X* Xlo = reinterpret_cast<X*>(cbase) + (it & 1) * (2 * L::XC + 2 * L::YC);
+    X* Xhi = Xlo + L::XC;
+    X* Ylo = Xhi + L::XC;
+    X* Yhi = Ylo + L::YC;
 
     // ---- register loads for this plane (prefetched) and the next one
     const P qe = qe_next;
-    R zr_hi = R(0), zl_hi = R(0);
+    X zlo_up = X();
+    typename Sw::F Fz_hi = typename Sw::F();
     if (!DIM2) {
       if (it + 1 < nplanes && fz_inb(A.err, gz, A.nfield)) qe_next = pmk(A.pi[gz], A.wi[gz]);
-      // ---- z: centre k+1
-      weno_waves<R>(qa, qb, qc, qd, qe, A.z0, zr_hi, zl_hi);
+      // ---- z: centre k+1 -> face k+1/2
+      X zhi_up;
+      Sw::centre(A, qa, qb, qc, qd, qe, zlo_up, zhi_up);
+      Fz_hi = Sw::face(A, zlo, zhi_up);
     }
 
     // ---- plane k tile
@@ -276,47 +295,46 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
                                                         !pml_xy && !pml_plane && fz_inb(A.err, gk, A.nfield));
 
     // ---- x and y centres of this thread's cell
-    R xr, xl, yr, yl;
+    X xlo, xhi, ylo, yhi;
     {
       const int c0 = (ty + HY) * PW + (tx + HX);
-      weno_waves<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
-                    pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), A.z0, xr, xl);
-      XR[ty * (TX + 2) + tx + 1] = xr;
-      XL[ty * (TX + 2) + tx + 1] = xl;
-      weno_waves<R>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]), pmk(Tp[c0], Tv[c0]),
-                    pmk(Tp[c0 + PW], Tv[c0 + PW]), pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, yr, yl);
-      YR[(ty + 1) * TX + tx] = yr;
-      YL[(ty + 1) * TX + tx] = yl;
+      Sw::centre(A, pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
+                 pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), xlo, xhi);
+      Xlo[ty * L::CP + tx + 1] = xlo;
+      Xhi[ty * L::CP + tx + 1] = xhi;
+      Sw::centre(A, pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]), pmk(Tp[c0], Tv[c0]),
+                 pmk(Tp[c0 + PW], Tv[c0 + PW]), pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), ylo, yhi);
+      Ylo[(ty + 1) * L::CP + tx] = ylo;
+      Yhi[(ty + 1) * L::CP + tx] = yhi;
     }
-    // ---- halo centres: warp 0 the x edges (wr of i0-1, wl of i0+TX) of all 16 rows, warps 1-2 the
-    //      y edge rows (wr of j0-1, wl of j0+TY)
+    // ---- halo centres: warp 0 the x edges (lo of i0-1, hi of i0+TX) of all 16 rows, warps 1-2 the
+    //      y edge rows (lo of j0-1, hi of j0+TY)
     if (lt < 2 * TY) {
       const int r = lt >> 1, side = lt & 1;
       const int c0 = (r + HY) * PW + (side ? (HX + TX) : (HX - 1));
-      R er, el;
-      weno_waves<R>(pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
-                    pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), A.z0, er, el);
+      X el, eh;
+      Sw::centre(A, pmk(Tp[c0 - 2], Tu[c0 - 2]), pmk(Tp[c0 - 1], Tu[c0 - 1]), pmk(Tp[c0], Tu[c0]),
+                 pmk(Tp[c0 + 1], Tu[c0 + 1]), pmk(Tp[c0 + 2], Tu[c0 + 2]), el, eh);
       if (side)
-        XL[r * (TX + 2) + TX + 1] = el;
+        Xhi[r * L::CP + TX + 1] = eh;
       else
-        XR[r * (TX + 2)] = er;
+        Xlo[r * L::CP] = el;
     } else if (lt >= 32 && lt < 32 + 2 * TX) {
       const int e = lt - 32;
       const int c = e & (TX - 1);
+      X el, eh;
       if (e < TX) {
         const int c0 = (HY - 1) * PW + (c + HX);
-        R er, unused;
-        weno_waves<R, WENO_LO>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
-                               pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
-                               pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, er, unused);
-        YR[c] = er;
+        Sw::template centre<WENO_LO>(A, pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
+                                     pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
+                                     pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), el, eh);
+        Ylo[c] = el;
       } else {
         const int c0 = (TY + HY) * PW + (c + HX);
-        R el, unused;
-        weno_waves<R, WENO_HI>(pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
-                               pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
-                               pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), A.z0, unused, el);
-        YL[(TY + 1) * TX + c] = el;
+        Sw::template centre<WENO_HI>(A, pmk(Tp[c0 - 2 * PW], Tv[c0 - 2 * PW]), pmk(Tp[c0 - PW], Tv[c0 - PW]),
+                                     pmk(Tp[c0], Tv[c0]), pmk(Tp[c0 + PW], Tv[c0 + PW]),
+                                     pmk(Tp[c0 + 2 * PW], Tv[c0 + 2 * PW]), el, eh);
+        Yhi[(TY + 1) * L::CP + c] = eh;
       }
     }
     // the per-plane barrier, with the OR of the threads' wait failures folded into it
@@ -335,16 +353,12 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       issue(it + 2);
     }
 
-    // ---- the RK update of this cell before its cPML and source terms: per direction the differences
-    //      X of wr and Y of wl across the cell (low minus high face), flux differences (times h)
-    //      c/2 (X - Y) for p and 1/(2 rho) (X + Y) for the velocity; then the stage combination
-    auto rk_update = [&](int64_t g, P& Dx, P& Dy, P& Dz, R& pn, R& un, R& vn, R& wn) {
-      const R Xx = XR[ty * (TX + 2) + tx] - xr, Yx = xl - XL[ty * (TX + 2) + tx + 2];
-      const R Xy = YR[ty * TX + tx] - yr, Yy = yl - YL[(ty + 2) * TX + tx];
-      const R Xz = zr_lo - zr, Yz = zl - zl_hi;
-      Dx = pmk(Xx - Yx, Xx + Yx);
-      Dy = pmk(Xy - Yy, Xy + Yy);
-      Dz = pmk(Xz - Yz, Xz + Yz);
+    // ---- the RK update of this cell before its cPML and source terms: differences across the cell
+    //      along each axis (.x pressure, .y velocity), stage combination
+    auto rk_update = [&](uint32_t g, P& Dx, P& Dy, P& Dz, R& pn, R& un, R& vn, R& wn) {
+      Dx = Sw::across(A, Xlo[ty * L::CP + tx], xhi, xlo, Xhi[ty * L::CP + tx + 2]);
+      Dy = Sw::across(A, Ylo[ty * L::CP + tx], yhi, ylo, Yhi[(ty + 2) * L::CP + tx]);
+      Dz = Sw::across(Fz_lo, Fz_hi);
       const int c0 = (ty + HY) * PW + (tx + HX);
       pn = fma(A.dt_p, (Dx.x + Dy.x) + Dz.x, DIM2 ? Tp[c0] : qb.x);
       un = fma(A.dt_v, Dx.y, Tu[c0]);
@@ -372,7 +386,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       A.vo[gk] = vn;
       A.wo[gk] = wn;
     } else if (valid && (cls & (CLS_UPDATE | CLS_SOURCE)) && fz_inb(A.err, gk, A.nfield)) {
-      const int64_t g = gk;
+      const uint32_t g = gk;
       if (cls & CLS_UPDATE) {
         P Dx, Dy, Dz;
         R pn, un, vn, wn;
@@ -396,9 +410,8 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       buf = 0;
       parity ^= 1u;
     }
-    zr_lo = zr;
-    zr = zr_hi;
-    zl = zl_hi;
+    Fz_lo = Fz_hi;
+    zlo = zlo_up;
     qa = qb;
     qb = qc;
     qc = qd;
@@ -435,28 +448,16 @@ __global__ void FZ_BAND_BOUNDS(R, KM) k_band(const __grid_constant__ BandArgs<R>
   band_body<R, STAGE, KM, LM, KEEP>(B, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Receiver gather after the last stage of a step (main3D.cu:1399-1414), into a device buffer;
-// then advances the device step counter. One block.
+// Receiver gather after the last stage of a step (main3D.cu:1399-1414), into a device buffer; then
+// advances the device step counter. One block. off: steps completed since the counter's value (those
+// before the last one were recorded by the stage 0 launches that followed them).
 template <class R>
 __device__ __forceinline__ void receivers_body(const R* __restrict__ p, const R* __restrict__ u,
                                                const R* __restrict__ v, const R* __restrict__ w,
                                                const int64_t* __restrict__ rcell, int nrec, double* ir, double* vel,
-                                               int64_t cap, int64_t* step, int32_t* err, int64_t nfield) {
-  const int64_t n = *step;
-  for (int r = threadIdx.x; r < nrec; r += blockDim.x) {
-    const int64_t c = rcell[r];
-    if (!fz_inb(err, c, nfield)) continue;
-    const double pp = (double)p[c], uu = (double)u[c], vv = (double)v[c], ww = (double)w[c];
-    // health word: a blown-up solution reaches the receivers (their samples are read anyway)
-    if (!isfinite(pp) || !isfinite(uu) || !isfinite(vv) || !isfinite(ww)) atomicOr(err, KERR_NONFINITE);
-    if (n < cap) {
-      const int64_t o = (int64_t)r * cap + n;
-      ir[o] = pp;
-      vel[3 * o + 0] = uu;
-      vel[3 * o + 1] = vv;
-      vel[3 * o + 2] = ww;
-    }
-  }
+                                               int64_t cap, int64_t* step, int off, int32_t* err, int64_t nfield) {
+  const int64_t n = *step + off;
+  record_samples<R>(p, u, v, w, rcell, nrec, ir, vel, cap, n, err, nfield, threadIdx.x, blockDim.x);
   __syncthreads();
   if (threadIdx.x == 0) *step = n + 1;
 }
@@ -464,8 +465,8 @@ __device__ __forceinline__ void receivers_body(const R* __restrict__ p, const R*
 template <class R>
 __global__ void k_receivers(const R* __restrict__ p, const R* __restrict__ u, const R* __restrict__ v,
                             const R* __restrict__ w, const int64_t* __restrict__ rcell, int nrec,
-                            double* ir, double* vel, int64_t cap, int64_t* step, int32_t* err, int64_t nfield) {
-  receivers_body<R>(p, u, v, w, rcell, nrec, ir, vel, cap, step, err, nfield);
+                            double* ir, double* vel, int64_t cap, int64_t* step, int off, int32_t* err, int64_t nfield) {
+  receivers_body<R>(p, u, v, w, rcell, nrec, ir, vel, cap, step, off, err, nfield);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -478,6 +479,7 @@ __global__ void k_receivers(const R* __restrict__ p, const R* __restrict__ u, co
 __shared__ int g_group_cta[3];  // tile coordinates of this CTA inside its room
 
 struct GroupCta {
+  static constexpr int planes = 1;
   static __device__ __forceinline__ int x() { return g_group_cta[0]; }
   static __device__ __forceinline__ int y() { return g_group_cta[1]; }
   static __device__ __forceinline__ int z() { return g_group_cta[2]; }
@@ -530,7 +532,7 @@ __global__ void FZ_BAND_BOUNDS(R, KM) k_band_group(const __grid_constant__ Group
 template <class R>
 __global__ void k_receivers_group(const RecArgs<R>* __restrict__ args) {
   const RecArgs<R>& a = args[blockIdx.x];
-  receivers_body<R>(a.p, a.u, a.v, a.w, a.rcell, a.nrec, a.ir, a.vel, a.cap, a.step, a.err, a.nfield);
+  receivers_body<R>(a.p, a.u, a.v, a.w, a.rcell, a.nrec, a.ir, a.vel, a.cap, a.step, 0, a.err, a.nfield);
 }
 
 // Non-finite values in a state (p, u, v, w over n cells), counted into *count.
@@ -708,7 +710,7 @@ cudaError_t launch_band(int stage, const BandArgs<R>& a, cudaStream_t s) {
   else if (fit == 4)                                                          \
     k_band<R, ST, 4, 4, KEEP><<<(unsigned)nb, bs, 0, s>>>(a);                 \
   else                                                                        \
-    k_band<R, ST, 0, 0, KEEP><<<(unsigned)nb, bs, 0, s>>>(a);
+    k_band<R, ST, 0, 0, true><<<(unsigned)nb, bs, 0, s>>>(a);
   if (stage == 0) {
     if (a.keep) { FZ_BAND_LAUNCH(0, true) } else { FZ_BAND_LAUNCH(0, false) }
   } else if (stage == 1) {
@@ -722,9 +724,9 @@ cudaError_t launch_band(int stage, const BandArgs<R>& a, cudaStream_t s) {
 
 template <class R>
 cudaError_t launch_receivers(const R* p, const R* u, const R* v, const R* w, const int64_t* rcell, int nrec,
-                             double* ir, double* vel, int64_t cap, int64_t* step, int32_t* err, int64_t nfield,
-                             cudaStream_t s) {
-  k_receivers<R><<<1, 256, 0, s>>>(p, u, v, w, rcell, nrec, ir, vel, cap, step, err, nfield);
+                             double* ir, double* vel, int64_t cap, int64_t* step, int off, int32_t* err,
+                             int64_t nfield, cudaStream_t s) {
+  k_receivers<R><<<1, 256, 0, s>>>(p, u, v, w, rcell, nrec, ir, vel, cap, step, off, err, nfield);
   return cudaGetLastError();
 }
 
@@ -799,7 +801,7 @@ cudaError_t launch_receivers_group(const RecArgs<R>* args, int n, cudaStream_t s
   template cudaError_t launch_stage<R>(int, bool, const StageArgs<R>&, const StageMaps&, dim3, cudaStream_t); \
   template cudaError_t launch_band<R>(int, const BandArgs<R>&, cudaStream_t);                      \
   template cudaError_t launch_receivers<R>(const R*, const R*, const R*, const R*, const int64_t*, \
-                                           int, double*, double*, int64_t, int64_t*, int32_t*,     \
+                                           int, double*, double*, int64_t, int64_t*, int, int32_t*, \
                                            int64_t, cudaStream_t);                                 \
   template cudaError_t launch_count_nonfinite<R>(const R*, const R*, const R*, const R*, int64_t,  \
                                                  unsigned long long*, int, cudaStream_t);         \

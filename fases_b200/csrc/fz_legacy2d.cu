@@ -32,6 +32,7 @@
 #include "fz_legacy2d.h"
 #include "fz_pair.cuh"
 #include "fz_wait.h"
+#include "fz_wave.h"
 
 namespace l2d {
 
@@ -54,7 +55,7 @@ struct Args {
   int Nx, Ny;
   R rho, c, dt;
   R eps;         // 3/4 of the scheme's (fz_pair.cuh)
-  R dt_p, dt_v;  // dt / h * c / 2, dt / h / (2 rho): per difference / sum of the characteristics
+  R z0, dt_p, dt_v;  // rho c; dt / h * c / 2, dt / h / (2 rho): per difference / sum of the characteristics
   const R *spx, *spy;  // sPML ramps along x and y
   const R* in[3];    // stage input p, u, v (stencils and probes)
   const R* base[3];  // U0 p, u, v (stages 1 and 2)
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(NT) k_l2d_stage(const Args<R> a) {
     b2 = a.base[2][C];
   }
   // centres: each once (WENO_x / WENO_y of functions.cuh:1125-1176)
-  const R Z0 = a.rho * a.c;
+  const R Z0 = a.z0;
   if (t < FX * TY) {
     const int row = t / FX, col = t % FX;  // node (i0 + col - 1, j0 + row)
     js_waves<R>(&sm[0][row + HALO][col + HALO - 1], &sm[1][row + HALO][col + HALO - 1], 1, a.eps, Z0, xw[0][row][col],
@@ -425,8 +426,7 @@ l2d::Args<R> args(fz_l2d* h, int stage, int par) {
   a.Nx = p.Nx; a.Ny = p.Ny;
   a.dt = (R)p.dt; a.rho = (R)p.rho; a.c = (R)p.c;
   a.eps = (R)(0.75 * p.eps);
-  a.dt_p = (R)(0.5 * p.dt * p.c / p.h);
-  a.dt_v = (R)(0.5 * p.dt / (p.h * p.rho));
+  fz::wave_constants(p.dt, p.c, p.h, p.rho, &a.z0, &a.dt_p, &a.dt_v);
   a.spx = (const R*)h->d_sp[0];
   a.spy = (const R*)h->d_sp[1];
   const int b0 = par, b1 = 1 - par;

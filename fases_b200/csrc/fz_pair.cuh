@@ -40,7 +40,6 @@ __device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) {
 }
 __device__ __forceinline__ double2 psub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 pabs(double2 a) { return make_double2(fabs(a.x), fabs(a.y)); }
-__device__ __forceinline__ double2 prcp(double2 a) { return make_double2(1.0 / a.x, 1.0 / a.y); }
 __device__ __forceinline__ double2 pswap(double2 a) { return make_double2(a.y, a.x); }
 
 template <class R>
@@ -49,38 +48,71 @@ __device__ __forceinline__ typename Pair<R>::T psplat(R x) {
 }
 
 // ------------------------------------------------------------------------------------------
-// WENO-Z reconstruction at one cell centre (Borges, Carmona, Costa & Don 2008, q = 1), the scheme
+// WENO reconstruction at one cell centre: WENO-Z (Borges, Carmona, Costa & Don 2008, q = 1), the scheme
 // of functions3D.cuh:763-1001 with the tables of main3D.cu:834-843 and eps = 1e-10 (main3D.cu:770).
 //
 // The reference evaluates V-(i+1/2) (idx = 1) and V+(i-1/2) (idx = 0) of a cell in two separate
 // calls; both use the same three smoothness indicators and the same factors (1 + tau/(beta+eps)),
-// and differ only in the linear weights d (mirrored) and the candidate rows. This evaluates them
-// together, on the first differences a..d of the five-point stencil. Multiplied out, the indicators
-// are quadratic forms of neighbouring differences,
-//   3/4 beta_2 = a^2 - 11/4 a b + 5/2 b^2    3/4 beta_1 = b^2 - 5/4 b c + c^2
-//   3/4 beta_0 = 5/2 c^2 - 11/4 c d + d^2
-// (each at least 0.6 of its larger square, so rounding cannot make one negative; the 3/4 goes into
-// eps), and the weighted candidates 5 d_r (V_r - u_i), scaled so that most coefficients are 1:
-//   V-: c - d/4, c + b/2, (5 b - 2 a)/12      V+: -(5 c - 2 d)/12, -(b + c/2), -(b - a/4)
-// with the normaliser 5 sum d_r q_r. 37 paired operations a centre for both faces, where second
-// differences and one-sided first derivatives as intermediates took 45; together with the exchange
-// of characteristics below, 500 x 400 x 200 cells in FP32: a stage 0.651 / 0.684 / 0.686 ms instead of
-// 0.694 / 0.731 / 0.733 (one z schedule, same box), IR error against 64 bits unchanged within the
-// scatter of seeds (0.86 to 1.08 of the former, geometric means over 12 seeds and 3 rooms).
+// and differ only in the linear weights d (mirrored) and the candidate rows. Both forms below evaluate
+// them together, on the first differences a..d of the five-point stencil.
 // ------------------------------------------------------------------------------------------
 // FACES selects the face values computed: WENO_BOTH, or only V- (WENO_LO) or V+ (WENO_HI) where a
 // caller uses one of them (the tile's halo rows); the value computed is the same either way.
 constexpr int WENO_LO = 1, WENO_HI = 2, WENO_BOTH = 3;
 
+// FP32, 3D solver: indicators from second differences D_r and one-sided first derivatives E_r,
+//   candidates:  u_i + delta_r,   V = u_i + sum_r w_r delta_r,   w_r = d_r q_r / sum d q
+//   12/13 beta_r = D_r^2 + 3/13 E_r^2
+// (the 12/13 scaling is absorbed into eps). 45 paired operations; the form below takes 37 and the
+// characteristics halve the exchange, 7 % of a large room's step, but another rounding than results
+// this library has given before: traces and fields keep their bits.
+template <int FACES = WENO_BOTH>
+__device__ __forceinline__ void weno_center(float2 qm2, float2 qm1, float2 q0, float2 qp1, float2 qp2, float2& vm,
+                                            float2& vp) {
+  auto K = [](double x) { return make_float2((float)x, (float)x); };
+  const float2 a = psub(qm1, qm2), b = psub(q0, qm1), c = psub(qp1, q0), d = psub(qp2, qp1);
+  const float2 D2 = psub(b, a), D1 = psub(c, b), D0 = psub(d, c);
+  const float2 E2 = pfma(b, K(2.0), D2);   // u_{i-2} - 4u_{i-1} + 3u_i
+  const float2 E1 = padd(b, c);            // -(u_{i-1} - u_{i+1})
+  const float2 E0 = pfma(c, K(-2.0), D0);  // 3u_i - 4u_{i+1} + u_{i+2} (sign)
+  const float2 k313 = K(3.0 / 13.0), eps = K(1e-10 * 12.0 / 13.0), one = K(1.0);
+  const float2 B0 = pfma(D0, D0, pfma(pmul(E0, k313), E0, eps));
+  const float2 B1 = pfma(D1, D1, pfma(pmul(E1, k313), E1, eps));
+  const float2 B2 = pfma(D2, D2, pfma(pmul(E2, k313), E2, eps));
+  const float2 tau = pabs(psub(B0, B2));
+  const float2 w0 = pfma(tau, prcp(B0), one);
+  const float2 w1 = pfma(tau, prcp(B1), one);
+  const float2 w2 = pfma(tau, prcp(B2), one);
+  // normalisers: V- uses d = (3/10, 3/5, 1/10), V+ the mirrored (1/10, 3/5, 3/10); d_r delta_r for
+  // both faces, written on the first and second differences
+  const float2 t1 = pmul(w1, K(0.6)), h1 = pmul(D1, K(0.05));
+  if constexpr ((FACES & WENO_LO) != 0) {
+    const float2 S = pfma(w0, K(0.3), pfma(w2, K(0.1), t1));
+    const float2 e0 = pfma(c, K(0.15), pmul(D0, K(-0.05)));
+    const float2 e1 = pfma(E1, K(0.15), h1);
+    const float2 e2 = pfma(b, K(0.05), pmul(D2, K(1.0 / 30.0)));
+    vm = pfma(pfma(w2, e2, pfma(w1, e1, pmul(w0, e0))), prcp(S), q0);
+  }
+  if constexpr ((FACES & WENO_HI) != 0) {
+    const float2 S = pfma(w0, K(0.1), pfma(w2, K(0.3), t1));
+    const float2 e0 = pfma(c, K(-0.05), pmul(D0, K(1.0 / 30.0)));
+    const float2 e1 = pfma(E1, K(-0.15), h1);
+    const float2 e2 = pfma(b, K(-0.15), pmul(D2, K(-0.05)));
+    vp = pfma(pfma(w2, e2, pfma(w1, e1, pmul(w0, e0))), prcp(S), q0);
+  }
+}
+
+// FP64, and the 2D legacy scheme: multiplied out, the indicators are quadratic forms of neighbouring
+// differences,
+//   3/4 beta_2 = a^2 - 11/4 a b + 5/2 b^2    3/4 beta_1 = b^2 - 5/4 b c + c^2
+//   3/4 beta_0 = 5/2 c^2 - 11/4 c d + d^2
+// (each at least 0.6 of its larger square, so rounding cannot make one negative; the 3/4 goes into
+// eps), and the weighted candidates 5 d_r (V_r - u_i), scaled so that most coefficients are 1:
+//   V-: c - d/4, c + b/2, (5 b - 2 a)/12      V+: -(5 c - 2 d)/12, -(b + c/2), -(b - a/4)
+// with the normaliser 5 sum d_r q_r: 37 operations a centre for both faces.
 // Nonlinear weights from the indicators B_r = 3/4 (beta_r + eps), up to a factor common to the three
 // (it cancels between the sums and their normalisers).
 struct WenoZ {  // 1 + tau / B_r, tau = |B_0 - B_2|
-  __device__ __forceinline__ void operator()(float2 B0, float2 B1, float2 B2, float2& w0, float2& w1, float2& w2) const {
-    const float2 tau = pabs(psub(B0, B2)), one = make_float2(1.f, 1.f);
-    w0 = pfma(tau, prcp(B0), one);
-    w1 = pfma(tau, prcp(B1), one);
-    w2 = pfma(tau, prcp(B2), one);
-  }
   // In FP64 a reciprocal costs several FMA-pipe operations: the factors times B_0 B_1 B_2
   __device__ __forceinline__ void operator()(double B0, double B1, double B2, double& w0, double& w1, double& w2) const {
     const double tau = fabs(B0 - B2);
@@ -193,12 +225,10 @@ __device__ __forceinline__ void weno_waves(typename Pair<R>::T qm2, typename Pai
   if constexpr ((FACES & WENO_HI) != 0) wl = fma(-Z0, fma(-Np.y, rp.y, q0.y), fma(-Np.x, rp.x, q0.x));
 }
 
-template <class R>
-__device__ __forceinline__ void weno_center(typename Pair<R>::T qm2, typename Pair<R>::T qm1, typename Pair<R>::T q0,
-                                            typename Pair<R>::T qp1, typename Pair<R>::T qp2, typename Pair<R>::T& vm,
-                                            typename Pair<R>::T& vp) {
-  typename Pair<R>::T Nm, Np, rm, rp;
-  weno_sums<WENO_BOTH>(qm2, qm1, q0, qp1, qp2, R(0.75e-10), WenoZ(), Nm, Np, rm, rp);
+__device__ __forceinline__ void weno_center(double2 qm2, double2 qm1, double2 q0, double2 qp1, double2 qp2, double2& vm,
+                                            double2& vp) {
+  double2 Nm, Np, rm, rp;
+  weno_sums<WENO_BOTH>(qm2, qm1, q0, qp1, qp2, 0.75e-10, WenoZ(), Nm, Np, rm, rp);
   vm = pfma(Nm, rm, q0);
   vp = psub(q0, pmul(Np, rp));
 }
@@ -212,5 +242,74 @@ __device__ __forceinline__ typename Pair<R>::T godunov(typename Pair<R>::T vm, t
   const typename Pair<R>::T sum = padd(vm, vp), dif = psub(vp, vm);
   return pfma(dif, kC, pmul(pswap(sum), kA));
 }
+
+// Difference of the Godunov fluxes through the low and the high face of a cell, F(lo) - F(hi),
+// from the face states (left state of a face = V- of the centre below it, right state = V+ of the
+// centre above): the flux is linear in the states, so the difference is taken on the sums and
+// differences first and swapped and scaled once.
+template <class R>
+__device__ __forceinline__ typename Pair<R>::T godunov_diff(typename Pair<R>::T vm_lo, typename Pair<R>::T vp_lo,
+                                                            typename Pair<R>::T vm_hi, typename Pair<R>::T vp_hi,
+                                                            typename Pair<R>::T kA, typename Pair<R>::T kC) {
+  const typename Pair<R>::T S = psub(padd(vm_lo, vp_lo), padd(vm_hi, vp_hi));
+  const typename Pair<R>::T D = psub(psub(vp_lo, vm_lo), psub(vp_hi, vm_hi));
+  return pfma(D, kC, pmul(pswap(S), kA));
+}
+
+// What the stage kernels pass between centres. A centre gives X lo for the face above it and X hi for
+// the face below; face() joins the lo of a centre and the hi of the one above it; the differences across
+// a cell (low minus high face) come as a (pressure, velocity) pair to be scaled by dt_p, dt_v.
+template <class R>
+struct Sweep;
+// FP32: both face states, and the flux differences of the states.
+template <>
+struct Sweep<float> {
+  typedef float2 X;
+  typedef float2 F;  // a face's flux
+  template <int FACES = WENO_BOTH, class A>
+  static __device__ __forceinline__ void centre(const A&, float2 qm2, float2 qm1, float2 q0, float2 qp1, float2 qp2,
+                                                X& lo, X& hi) {
+    weno_center<FACES>(qm2, qm1, q0, qp1, qp2, lo, hi);
+  }
+  template <class A>
+  static __device__ __forceinline__ F face(const A& a, X lo, X hi) {
+    return godunov<float>(lo, hi, pmk(a.frc2, a.firho), psplat<float>(-a.fc));
+  }
+  static __device__ __forceinline__ float2 across(F below, F above) { return psub(below, above); }
+  // from the states: lo of the centre below, own hi, own lo, hi of the centre above
+  template <class A>
+  static __device__ __forceinline__ float2 across(const A& a, X lo_below, X hi, X lo, X hi_above) {
+    return godunov_diff<float>(lo_below, hi, lo, hi_above, pmk(a.frc2, a.firho), psplat<float>(-a.fc));
+  }
+};
+// FP64: the characteristics wr, wl. (X - Y, X + Y) of their differences.
+template <>
+struct Sweep<double> {
+  typedef double X;
+  typedef double2 F;  // (wr of the centre below, wl of the centre above)
+  template <int FACES = WENO_BOTH, class A>
+  static __device__ __forceinline__ void centre(const A& a, double2 qm2, double2 qm1, double2 q0, double2 qp1,
+                                                double2 qp2, X& lo, X& hi) {
+    weno_waves<double, FACES>(qm2, qm1, q0, qp1, qp2, a.z0, lo, hi);
+  }
+  template <class A>
+  static __device__ __forceinline__ F face(const A&, X lo, X hi) {
+    return make_double2(lo, hi);
+  }
+  static __device__ __forceinline__ double2 across(F below, F above) {
+    const double x = below.x - above.x, y = below.y - above.y;
+    return make_double2(x - y, x + y);
+  }
+  template <class A>
+  static __device__ __forceinline__ double2 across(const A&, X lo_below, X hi, X lo, X hi_above) {
+    return across(make_double2(lo_below, hi), make_double2(lo, hi_above));
+  }
+};
+__device__ __forceinline__ float shfl_up1(float x) { return __shfl_up_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ float2 shfl_up1(float2 x) { return make_float2(shfl_up1(x.x), shfl_up1(x.y)); }
+__device__ __forceinline__ double shfl_up1(double x) { return __shfl_up_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ float shfl_down1(float x) { return __shfl_down_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ float2 shfl_down1(float2 x) { return make_float2(shfl_down1(x.x), shfl_down1(x.y)); }
+__device__ __forceinline__ double shfl_down1(double x) { return __shfl_down_sync(0xffffffffu, x, 1); }
 
 }  // namespace fz
