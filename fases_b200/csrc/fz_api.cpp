@@ -97,6 +97,8 @@ void free_device(fz_handle* h) {
   dfree(h->d_ir);
   dfree(h->d_vel);
   dfree(h->d_slices);
+  dfree(h->d_pack);
+  h->pack_bytes = 0;
   h->sl_on = false;
 }
 
@@ -898,25 +900,70 @@ int load_geometry(fz_handle* h, const float* S, const uint8_t* oid, int Nx, int 
   return FZ_OK;
 }
 
+constexpr size_t PACK_KEEP = (size_t)32 << 20;
+
+// The requested fields, packed on the device into a workspace (all of them at once while that is
+// small, else one field of one member at a time), copied in one piece and widened on the host; FP64
+// values go straight into the caller's arrays.
 template <class R>
 int get_fields(fz_handle* h, double* p, double* u, double* v, double* w) {
-  const size_t rowb = (size_t)h->Nx * sizeof(R);
-  const size_t N = (size_t)h->Nx * h->Ny * h->Nz;
-  std::vector<R> tmp(N);
+  const int64_t N = (int64_t)h->Nx * h->Ny * h->Nz, per = N * h->nb;
   double* outs[4] = {p, u, v, w};
-  for (int f = 0; f < 4; f++) {
-    if (!outs[f]) continue;
-    for (int m = 0; m < h->nb; m++) {
-      const R* src = (const R*)h->U[h->i0][f] + XOFF + (size_t)m * h->ncell_dev;
-      FZ_CUDA(h, cudaMemcpy2D(tmp.data(), rowb, src, (size_t)h->Sx * sizeof(R), rowb,
-                              (size_t)h->Ny * h->Nz, cudaMemcpyDeviceToHost), "fields D2H");
-      double* o = outs[f] + (size_t)m * N;
-      const R* t = tmp.data();
-#pragma omp parallel for schedule(static)
-      for (int64_t c = 0; c < (int64_t)N; c++) o[c] = (double)t[c];
-    }
+  std::vector<int> want;
+  for (int f = 0; f < 4; f++)
+    if (outs[f]) want.push_back(f);
+  if (want.empty()) return FZ_OK;
+  const bool small = want.size() * (size_t)per * sizeof(R) <= PACK_KEEP;
+  const size_t bytes = small ? want.size() * (size_t)per * sizeof(R) : (size_t)N * sizeof(R);
+  if (h->pack_bytes < bytes) {
+    dfree(h->d_pack);
+    h->pack_bytes = 0;
+    FZ_CUDA(h, cudaMalloc(&h->d_pack, bytes), "cudaMalloc(field pack)");
+    h->pack_bytes = bytes;
   }
-  return FZ_OK;
+  if (sizeof(R) == 4 && h->pack_host.size() < bytes) h->pack_host.resize(bytes);
+  auto move = [&](const int* fields, int nf, int64_t member, int64_t members) -> int {
+    fz::PackArgs<R> a{};
+    for (int q = 0; q < nf; q++) a.src[q] = (const R*)h->U[h->i0][fields[q]] + XOFF + member * h->ncell_dev;
+    a.dst = (R*)h->d_pack;
+    a.rows = (int64_t)h->Ny * h->Nz * members;
+    a.Nx = h->Nx;
+    a.Sx = h->Sx;
+    a.nf = nf;
+    const int64_t n = N * members;
+    FZ_CUDA(h, fz::launch_pack<R>(a, h->nsm, h->stream), "field pack");
+    if (sizeof(R) == 8) {
+      for (int q = 0; q < nf; q++)
+        FZ_CUDA(h, cudaMemcpyAsync(outs[fields[q]] + member * N, (R*)h->d_pack + q * n, (size_t)n * sizeof(R),
+                                   cudaMemcpyDeviceToHost, h->stream), "fields D2H");
+      FZ_CUDA(h, cudaStreamSynchronize(h->stream), "fields D2H");
+      return FZ_OK;
+    }
+    FZ_CUDA(h, cudaMemcpyAsync(h->pack_host.data(), h->d_pack, (size_t)n * nf * sizeof(R), cudaMemcpyDeviceToHost,
+                               h->stream), "fields D2H");
+    FZ_CUDA(h, cudaStreamSynchronize(h->stream), "fields D2H");
+    const R* t = (const R*)h->pack_host.data();
+    for (int q = 0; q < nf; q++) {
+      double* o = outs[fields[q]] + member * N;
+      const R* f = t + q * n;
+#pragma omp parallel for schedule(static) if (n > 100000)
+      for (int64_t c = 0; c < n; c++) o[c] = (double)f[c];
+    }
+    return FZ_OK;
+  };
+  int rc = FZ_OK;
+  if (small) {
+    rc = move(want.data(), (int)want.size(), 0, h->nb);
+  } else {
+    for (size_t q = 0; q < want.size() && rc == FZ_OK; q++)
+      for (int m = 0; m < h->nb && rc == FZ_OK; m++) rc = move(&want[q], 1, m, 1);
+  }
+  if (bytes > PACK_KEEP) {
+    dfree(h->d_pack);
+    h->pack_bytes = 0;
+    std::vector<char>().swap(h->pack_host);
+  }
+  return rc;
 }
 
 template <class R>

@@ -219,6 +219,15 @@ struct DirectArgs {
   const int32_t* bidx;
 };
 
+// Fields packed for the host (k_pack): nf fields of `rows` rows of Nx elements, row pitch Sx.
+template <class R>
+struct PackArgs {
+  const R* src[4];
+  R* dst;
+  int64_t rows, Nx, Sx;
+  int32_t nf;
+};
+
 // Receiver gather of one room (the arguments of its receiver kernel).
 template <class R>
 struct RecArgs {

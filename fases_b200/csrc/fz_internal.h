@@ -110,6 +110,10 @@ struct fz_handle {
   int32_t* d_err = nullptr;
 
   // step counter and bookkeeping
+  // workspaces of fz_get_fields, kept while they are small (PACK_KEEP bytes)
+  void* d_pack = nullptr;
+  size_t pack_bytes = 0;
+  std::vector<char> pack_host;
   int64_t* d_step = nullptr;
   double* d_scratch = nullptr;
   int64_t steps_enqueued = 0;

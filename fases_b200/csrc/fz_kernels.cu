@@ -535,6 +535,18 @@ __global__ void k_receivers_group(const RecArgs<R>* __restrict__ args) {
   receivers_body<R>(a.p, a.u, a.v, a.w, a.rcell, a.nrec, a.ir, a.vel, a.cap, a.step, 0, a.err, a.nfield);
 }
 
+// Rows of up to four padded fields packed without their padding, one field after another: dst[f][row][i].
+// One contiguous copy to the host then replaces a strided one per field, whose short rows (a few
+// hundred bytes) the copy engine takes one by one.
+template <class R>
+__global__ void k_pack(PackArgs<R> A) {
+  const int64_t n = A.rows * A.Nx, total = n * A.nf;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t f = c / n, e = c - f * n, row = e / A.Nx;
+    A.dst[c] = A.src[f][A.Sx * row + (e - row * A.Nx)];
+  }
+}
+
 // Non-finite values in a state (p, u, v, w over n cells), counted into *count.
 template <class R>
 __global__ void k_count_nonfinite(const R* __restrict__ p, const R* __restrict__ u, const R* __restrict__ v,
@@ -731,6 +743,14 @@ cudaError_t launch_receivers(const R* p, const R* u, const R* v, const R* w, con
 }
 
 template <class R>
+cudaError_t launch_pack(const PackArgs<R>& a, int nsm, cudaStream_t s) {
+  const int64_t blocks = (a.rows * a.Nx * a.nf + 255) / 256;
+  if (blocks <= 0) return cudaSuccess;
+  k_pack<R><<<(unsigned)(blocks < nsm * 8 ? blocks : nsm * 8), 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+template <class R>
 cudaError_t launch_count_nonfinite(const R* p, const R* u, const R* v, const R* w, int64_t n,
                                    unsigned long long* count, int nsm, cudaStream_t s) {
   k_count_nonfinite<R><<<nsm * 8, 256, 0, s>>>(p, u, v, w, n, count);
@@ -803,6 +823,7 @@ cudaError_t launch_receivers_group(const RecArgs<R>* args, int n, cudaStream_t s
   template cudaError_t launch_receivers<R>(const R*, const R*, const R*, const R*, const int64_t*, \
                                            int, double*, double*, int64_t, int64_t*, int, int32_t*, \
                                            int64_t, cudaStream_t);                                 \
+  template cudaError_t launch_pack<R>(const PackArgs<R>&, int, cudaStream_t);                      \
   template cudaError_t launch_count_nonfinite<R>(const R*, const R*, const R*, const R*, int64_t,  \
                                                  unsigned long long*, int, cudaStream_t);         \
   template cudaError_t launch_slices<R>(const R*, const R*, const R*, const R*, int, int, int, int64_t, int, int, \

@@ -32,6 +32,8 @@ cudaError_t launch_receivers(const R* p, const R* u, const R* v, const R* w, con
                              int nrec, double* ir, double* vel, int64_t cap, int64_t* step, int off, int32_t* err,
                              int64_t nfield, cudaStream_t s);
 template <class R>
+cudaError_t launch_pack(const PackArgs<R>& a, int nsm, cudaStream_t s);
+template <class R>
 cudaError_t launch_count_nonfinite(const R* p, const R* u, const R* v, const R* w, int64_t n,
                                    unsigned long long* count, int nsm, cudaStream_t s);
 template <class R>
