@@ -60,3 +60,56 @@ def test_direct_kernel_equals_marching_kernel(case, precision):
     for x, y in zip(a, b):
         assert np.isfinite(x).all() and np.abs(a[0]).max() > 0
         assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("depth", [0, 3])  # the direct and the marching kernel
+def test_samples_of_a_run_equal_those_of_single_steps(depth, precision):
+    """A run records the samples of all but its last step in the stage launch that follows, and
+    advances the step counter once (per graph, and per 16 steps beyond); single steps record each
+    by the receiver kernel. Lengths around the graph (10) and the direct sequence (16); the source
+    waveform follows the step either way."""
+    h, c, rho, steps = 0.05, 343.0, 1.2, 47
+    rng = np.random.default_rng(8)
+    dt = 0.5 * h / c
+    sc = scenes.box_room((33, 21, 17), h)
+    m = mats.pack([mats.random_passive(rng, dt, c / (4 * h)) for _ in range(6)])
+
+    def solve(parts):
+        s = Solver(params(h=h, c=c, rho=rho, dt=dt, precision=precision))
+        s.load_geometry(sc.S, sc.oid)
+        s.set_materials(m["Rinf"], m["A"], m["zeta"], m["B"], m["Cc"], m["alpha"], m["beta"])
+        s.set_sources(np.array([[12, 11, 10]], np.int32), np.array([1e-3]), 0, u_s=np.sin(0.3 * np.arange(2 * steps + 3)))
+        s.set_receivers(np.array([[15, 11, 10], [30, 18, 5]], np.int32), steps)
+        if depth:
+            s.set_kz_chunk(depth)
+        for n in parts:
+            s.run(n)
+        assert s.steps_done() == steps
+        out = s.ir(), s.vel()
+        s.close()
+        return out
+
+    one = solve([1] * steps)
+    for parts in ([steps], [9, 10, 11, 17], [2, 45]):
+        for x, y in zip(one, solve(parts)):
+            assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("room,batch", [((9, 5, 4), 1), ((31, 17, 6), 3), ((140, 131, 117), 1), ((90, 80, 75), 4)])
+def test_fields_come_back_as_they_were_set(room, batch, precision):
+    """fz_get_fields packs the fields on the device: all at once while they are small (32 MB), else one
+    field of one member at a time."""
+    sc = scenes.box_room(room, 0.05)
+    s = Solver(params(h=0.05, precision=precision, batch=batch))
+    s.load_geometry(sc.S, sc.oid)
+    rng = np.random.default_rng(3)
+    shape = ((batch,) if batch > 1 else ()) + sc.shape
+    f = [rng.standard_normal(shape) for _ in range(4)]
+    s.set_fields(*f)
+    for got, want in zip(s.fields(), f):
+        assert np.array_equal(got, want.astype(np.float32) if precision == "fp32" else want)
+    s.close()
