@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(ANTHREADS, 1) k_adj_stage(const AdjStageArgs<R
   }
   uint8_t prc[NE];
   // plane k into raw buffer k & 1, asynchronously (zeros outside the grid); the class bytes, too small
-  // for an asynchronous copy, pass through a register
+  // for an asynchronous copy, pass through a register. (Through registers, the twelve values a thread
+  // holds across the iteration made the FP64 kernel spill 420 instead of 212 bytes.)
   auto prefetch = [&](int k) {
     R* raw = sm + (k & 1) * S::RAW;
 #pragma unroll
@@ -661,13 +662,33 @@ __global__ void __launch_bounds__(256) k_adj_grad_reduce(const int4* rec, const 
     if (bins[m] != 0.0) atomicAdd(&grad[(int64_t)m * P + e], bins[m]);
 }
 
+// The traces' adjoint, added at the receiver cells by one warp. Receivers may share a cell: a warp
+// whose cells differ adds at once (16 receivers one after another took 11 us of chained loads), else
+// lane by lane, in receiver order either way.
 template <class R>
-__global__ void k_adj_receivers(R* lp, const int64_t* rcell, int nrec, const double* ir, int64_t cap,
-                                const double* target, int64_t tlen, int64_t n, int cotangent) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int r = 0; r < nrec; r++) {  // one thread: receivers may share a cell
-    const double t = target[(int64_t)r * tlen + n];
-    lp[rcell[r]] += (R)(cotangent ? t : 2.0 * (ir[(int64_t)r * cap + n] - t));
+__global__ void __launch_bounds__(32) k_adj_receivers(R* lp, const int64_t* rcell, int nrec, const double* ir,
+                                                      int64_t cap, const double* target, int64_t tlen, int64_t n,
+                                                      int cotangent) {
+  const int lane = threadIdx.x;
+  for (int r0 = 0; r0 < nrec; r0 += 32) {
+    const int r = r0 + lane;
+    const bool on = r < nrec;
+    const unsigned long long c = on ? (unsigned long long)rcell[r] : ~0ull - lane;  // idle lanes: values of their own
+    R add = R(0);
+    if (on) {
+      const double t = target[(int64_t)r * tlen + n];
+      add = (R)(cotangent ? t : 2.0 * (ir[(int64_t)r * cap + n] - t));
+    }
+    const bool alone = __popc(__match_any_sync(0xffffffffu, c)) == 1;
+    if (__all_sync(0xffffffffu, alone)) {
+      if (on) lp[c] += add;
+    } else {
+      for (int q = 0; q < 32; q++) {
+        if (on && lane == q) lp[c] += add;
+        __syncwarp();
+      }
+    }
+    __syncwarp();
   }
 }
 
