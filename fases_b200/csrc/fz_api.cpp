@@ -370,10 +370,11 @@ int build_band(fz_handle* h) {
 
 // Whether the room runs the direct stage kernel (fz_direct.cu): while its warps, 30 cells of a row
 // each, come to at most two waves of what the GPU holds (16 per SM). Measured, us a step, direct /
-// marching at its best chunk depth: 3D FP32 26 x 22 x 18 (396 warps) 17 / 29, 45 x 38 x 29 (2204) 20 / 33,
-// 71 x 53 x 47 (7473) 49 / 46, 96^3 182 / 93; FP64 18 / 35, 31 / 43, 65 / 65, 283 / 174. A planar room's
-// direct kernel has no redundant centres to pay for, so it goes a little further: FP32 256 x 256 (2304)
-// 18 / 29, 500 x 400 (6800) 36 / 35, FP64 25 / 33, 44 / 50, 800 x 800 (21600) 125 / 113.
+// marching with chunks chosen for latency: 3D FP32 26 x 22 x 18 (396 warps) 15 / 27, 45 x 38 x 29 (2204)
+// 19 / 31, 58 x 46 x 40 (3680) 30 / 33, 71 x 53 x 47 (7473) 49 / 45, 64^3 69 / 45; FP64 19 / 31, 26 / 41,
+// 40 / 40, 70 / 60, 101 / 60. A planar room's direct kernel has no redundant centres to pay for, so it
+// goes a little further: FP32 256 x 256 (2304) 16 / 26, 500 x 400 (6800) 34 / 33, 800 x 800 104 / 60; FP64
+// 19 / 33, 44 / 50, 125 / 113.
 template <class R>
 bool use_direct(const fz_handle* h) {
 #ifdef FZ_WAIT_TEST

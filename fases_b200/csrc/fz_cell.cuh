@@ -154,7 +154,10 @@ __device__ __forceinline__ void ade_pair(double& r1, double& r2, double m1, doub
 // middle sets. Otherwise only the last stage stores states: the recursion is linear in the state at
 // step start and the outgoing characteristics, so stages 1 and 2 recompute the earlier stages' states
 // from those (8 bytes a stage, kept in wst) instead of reading and writing sets of 8 (K + 2L) bytes.
-// With K = L = 2 a band cell moves 176 instead of 384 bytes of states a step, with the same bits.
+// With K = L = 2 a band cell moves 176 instead of 384 bytes of states a step, with the same bits:
+// 500 x 400 x 200 cells (2.35 M band cells) 120 us a launch instead of 137, 190 x 150 x 140 FP64 39
+// instead of 44. By its counters (192^3) the kernel then reads 231 bytes of DRAM a cell and launch, 58 %
+// of the copy rate: band rows of walls normal to x are three cells long, a third of a sector.
 // KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
 // probe is then issued at the top, beside the probe gathers, so one thread keeps ~50 loads in flight;
 // KM = LM = 0 is the general form with the state loads inside the pole loops; it keeps every state.

@@ -2,10 +2,11 @@
 //
 // One SSP-RK3 step of the reference (3D-solver/core/main3D.cu:1280-1319) is nine launches there:
 // three stage kernels (functions3D.cuh:1086-1327), three source injections (1039-1047) and three
-// full-grid immersed-boundary passes (462-565). Here it is seven: three fused stage kernels
-// (WENO-Z reconstruction once per face, Godunov flux, RK combination, cPML and source injection
-// in one pass), three sparse band kernels that touch only the immersed band cells, and one
-// receiver gather.
+// full-grid immersed-boundary passes (462-565). Here it is six: three fused stage kernels (WENO-Z
+// reconstruction once per face, Godunov flux, RK combination, cPML and source injection in one
+// pass; stage 0 also records the receiver samples of the step before it) and three sparse band
+// kernels that touch only the immersed band cells; a receiver gather ends each run of steps. Small
+// rooms run three (fz_direct.cu).
 #include <cuda_runtime.h>
 #include <math.h>
 
