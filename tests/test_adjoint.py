@@ -180,3 +180,30 @@ def test_adjoint_other_pole_counts(K, L):
         assert abs(fd - gval) <= 1e-3 * abs(fd), (K, L, name, gval, fd)
         checked += 1
     assert checked >= 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("copies", [1, 2, 8, 17])
+def test_receivers_that_share_cells_add_up(copies):
+    """The reverse sweep is linear in the traces' adjoint, so receivers placed several times over with
+    targets of their own give the sum of the gradients they give one set at a time (4 to 68
+    receivers: within and across the warp that adds them, all apart or sharing cells)."""
+    cfg = _cfg()
+    base = np.asarray(cfg["recs"])
+    rng = np.random.default_rng(8)
+    targets = [1e-3 * rng.standard_normal((len(base), STEPS)) for _ in range(copies)]
+
+    def grad(recs, target):
+        s = _solver(dict(cfg, recs=np.ascontiguousarray(recs)), "fp64")
+        g = s.misfit_gradient(target, segment_steps=16)
+        s.close()
+        return g
+
+    whole = grad(np.concatenate([base] * copies), np.concatenate(targets))
+    parts = [grad(base, t) for t in targets]
+    for key in KEYS:
+        want = sum(np.asarray(p[key]) for p in parts)
+        # rounding of the same sums in another order (the probe scatter adds with atomics): 1e-16 a term
+        # over some 1e3 terms and the sweep's growth
+        scale = sum(np.abs(np.asarray(p[key])).max() for p in parts)
+        assert np.abs(np.asarray(whole[key]) - want).max() <= 1e-10 * scale, key
