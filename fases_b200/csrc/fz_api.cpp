@@ -901,70 +901,76 @@ int load_geometry(fz_handle* h, const float* S, const uint8_t* oid, int Nx, int 
   return FZ_OK;
 }
 
-constexpr size_t PACK_KEEP = (size_t)32 << 20;
+constexpr size_t PACK_BYTES = (size_t)4 << 20;  // most of the field pack, on the device and the host
 
-// The requested fields, packed on the device into a workspace (all of them at once while that is
-// small, else one field of one member at a time), copied in one piece and widened on the host; FP64
-// values go straight into the caller's arrays.
+// The requested fields, packed on the device into a workspace (all of them at once where they fit, else
+// slabs of one field's rows), copied in one piece into a kept host buffer and widened or copied from there
+// by all threads (a fresh array's pages are then mapped in parallel, not by the one thread of the device
+// copy). 256 x 256 FP64 plane: 2.4 ms, row by row without the pack 3.5, straight into the caller's arrays
+// 7.2. At 1 MB it is 2.9 to 3.4; at 16 and 32 MB 2.3, but mapping the buffer costs the first call 4 ms more.
+// A device without room for the workspace copies the padded rows one by one.
 template <class R>
 int get_fields(fz_handle* h, double* p, double* u, double* v, double* w) {
-  const int64_t N = (int64_t)h->Nx * h->Ny * h->Nz, per = N * h->nb;
+  const int64_t Nx = h->Nx, rows = (int64_t)h->Ny * h->Nz * h->nb;  // members follow one another
   double* outs[4] = {p, u, v, w};
-  std::vector<int> want;
+  int want[4], nw = 0;
   for (int f = 0; f < 4; f++)
-    if (outs[f]) want.push_back(f);
-  if (want.empty()) return FZ_OK;
-  const bool small = want.size() * (size_t)per * sizeof(R) <= PACK_KEEP;
-  const size_t bytes = small ? want.size() * (size_t)per * sizeof(R) : (size_t)N * sizeof(R);
+    if (outs[f]) want[nw++] = f;
+  if (nw == 0) return FZ_OK;
+  const size_t rowb = (size_t)Nx * sizeof(R), all = (size_t)rows * rowb * nw;
+  const size_t bytes = std::min(all, std::max(PACK_BYTES, rowb));
   if (h->pack_bytes < bytes) {
     dfree(h->d_pack);
     h->pack_bytes = 0;
-    FZ_CUDA(h, cudaMalloc(&h->d_pack, bytes), "cudaMalloc(field pack)");
-    h->pack_bytes = bytes;
+    if (cudaMalloc(&h->d_pack, bytes) == cudaSuccess) {
+      h->pack_bytes = bytes;
+    } else {
+      h->d_pack = nullptr;
+      cudaGetLastError();
+    }
   }
-  if (sizeof(R) == 4 && h->pack_host.size() < bytes) h->pack_host.resize(bytes);
-  auto move = [&](const int* fields, int nf, int64_t member, int64_t members) -> int {
+  const bool pack = h->d_pack != nullptr;
+  if (h->pack_host_bytes < bytes) {
+    h->pack_host.reset(new (std::nothrow) char[bytes]);  // not cleared
+    h->pack_host_bytes = h->pack_host ? bytes : 0;
+    if (!h->pack_host) return set_error(h, FZ_ENOMEM, "fz_get_fields: out of host memory");
+  }
+  // rows [r0, r0 + n) of nf fields
+  auto move = [&](const int* fields, int nf, int64_t r0, int64_t n) -> int {
+    const size_t cells = (size_t)(n * Nx);
     fz::PackArgs<R> a{};
-    for (int q = 0; q < nf; q++) a.src[q] = (const R*)h->U[h->i0][fields[q]] + XOFF + member * h->ncell_dev;
+    for (int q = 0; q < nf; q++) a.src[q] = (const R*)h->U[h->i0][fields[q]] + XOFF + r0 * h->Sx;
     a.dst = (R*)h->d_pack;
-    a.rows = (int64_t)h->Ny * h->Nz * members;
+    a.rows = n;
     a.Nx = h->Nx;
     a.Sx = h->Sx;
     a.nf = nf;
-    const int64_t n = N * members;
-    FZ_CUDA(h, fz::launch_pack<R>(a, h->nsm, h->stream), "field pack");
-    if (sizeof(R) == 8) {
-      for (int q = 0; q < nf; q++)
-        FZ_CUDA(h, cudaMemcpyAsync(outs[fields[q]] + member * N, (R*)h->d_pack + q * n, (size_t)n * sizeof(R),
-                                   cudaMemcpyDeviceToHost, h->stream), "fields D2H");
-      FZ_CUDA(h, cudaStreamSynchronize(h->stream), "fields D2H");
-      return FZ_OK;
-    }
-    FZ_CUDA(h, cudaMemcpyAsync(h->pack_host.data(), h->d_pack, (size_t)n * nf * sizeof(R), cudaMemcpyDeviceToHost,
-                               h->stream), "fields D2H");
-    FZ_CUDA(h, cudaStreamSynchronize(h->stream), "fields D2H");
-    const R* t = (const R*)h->pack_host.data();
+    if (pack) FZ_CUDA(h, fz::launch_pack<R>(a, h->nsm, h->stream), "field pack");
     for (int q = 0; q < nf; q++) {
-      double* o = outs[fields[q]] + member * N;
-      const R* f = t + q * n;
-#pragma omp parallel for schedule(static) if (n > 100000)
-      for (int64_t c = 0; c < n; c++) o[c] = (double)f[c];
+      R* to = (R*)h->pack_host.get() + q * cells;
+      if (!pack)
+        FZ_CUDA(h, cudaMemcpy2DAsync(to, rowb, a.src[q], (size_t)h->Sx * sizeof(R), rowb, (size_t)n,
+                                     cudaMemcpyDeviceToHost, h->stream), "fields D2H");
+      else if (q == 0)
+        FZ_CUDA(h, cudaMemcpyAsync(to, a.dst, cells * nf * sizeof(R), cudaMemcpyDeviceToHost, h->stream), "fields D2H");
+    }
+    FZ_CUDA(h, cudaStreamSynchronize(h->stream), "fields D2H");
+    for (int q = 0; q < nf; q++) {
+      double* o = outs[fields[q]] + r0 * Nx;
+      const R* f = (const R*)h->pack_host.get() + q * cells;
+#pragma omp parallel for schedule(static) if (cells > 100000)
+      for (int64_t c = 0; c < (int64_t)cells; c++) o[c] = (double)f[c];
     }
     return FZ_OK;
   };
-  int rc = FZ_OK;
-  if (small) {
-    rc = move(want.data(), (int)want.size(), 0, h->nb);
-  } else {
-    for (size_t q = 0; q < want.size() && rc == FZ_OK; q++)
-      for (int m = 0; m < h->nb && rc == FZ_OK; m++) rc = move(&want[q], 1, m, 1);
-  }
-  if (bytes > PACK_KEEP) {
-    dfree(h->d_pack);
-    h->pack_bytes = 0;
-    std::vector<char>().swap(h->pack_host);
-  }
-  return rc;
+  if (all <= bytes) return move(want, nw, 0, rows);
+  const int64_t slab = (int64_t)(bytes / rowb);
+  for (int q = 0; q < nw; q++)
+    for (int64_t r0 = 0; r0 < rows; r0 += slab) {
+      const int rc = move(&want[q], 1, r0, std::min(slab, rows - r0));
+      if (rc != FZ_OK) return rc;
+    }
+  return FZ_OK;
 }
 
 template <class R>

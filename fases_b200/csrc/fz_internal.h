@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -113,7 +114,8 @@ struct fz_handle {
   // workspaces of fz_get_fields, kept while they are small (PACK_KEEP bytes)
   void* d_pack = nullptr;
   size_t pack_bytes = 0;
-  std::vector<char> pack_host;
+  std::unique_ptr<char[]> pack_host;  // pack_host_bytes
+  size_t pack_host_bytes = 0;
   int64_t* d_step = nullptr;
   double* d_scratch = nullptr;
   int64_t steps_enqueued = 0;

@@ -101,8 +101,8 @@ def test_samples_of_a_run_equal_those_of_single_steps(depth, precision):
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 @pytest.mark.parametrize("room,batch", [((9, 5, 4), 1), ((31, 17, 6), 3), ((140, 131, 117), 1), ((90, 80, 75), 4)])
 def test_fields_come_back_as_they_were_set(room, batch, precision):
-    """fz_get_fields packs the fields on the device: all at once while they are small (32 MB), else one
-    field of one member at a time."""
+    """fz_get_fields packs the fields on the device: all at once while they are small (4 MB), else slabs
+    of one field's rows, which may cross members."""
     sc = scenes.box_room(room, 0.05)
     s = Solver(params(h=0.05, precision=precision, batch=batch))
     s.load_geometry(sc.S, sc.oid)
