@@ -256,6 +256,9 @@ int fz_group_set_branches(fz_group* g, int32_t branches);
  * stage kernels' time per step; fz_get_z_schedule lists the chunks. fz_group_autotune does the
  * same for all members at once, timing their kernels side by side with one uniform depth for every
  * member (clamped to each room; 0 = each member's heuristic). Results do not depend on the depth (each CTA recomputes its boundary centres).
+ * Small rooms run a kernel without chunks (stage and band in one launch) unless a depth or schedule is
+ * set; where that applies the trials time stage and band kernels and it is one of the candidates; when it
+ * wins, kz_chunk is the heuristic depth, and another handle gets the same kernel by depth 0.
  * The reference launches fixed TP(32,4,4) blocks (main3D.cu:1280-1306). */
 int fz_autotune(fz_handle* h, int32_t reps, int32_t* kz_chunk, double* ms_per_step);
 int fz_group_autotune(fz_group* g, int32_t reps, int32_t* kz_chunk, double* ms_per_step);
