@@ -1,0 +1,30 @@
+"""The WENO centres over the range of their types. Smoothness indicators lie between eps and the square of
+the largest difference, and the weights are formed from products of them: a very small eps (the 2D
+legacy scheme takes any positive one) or very large fields must not carry those products out of the
+type's range. Against the CPU oracle, which divides; FP64 to 1e-10 and FP32 to 1e-5, the tolerances of
+the ordinary parity tests (a relative perturbation of 1e-15 of the start moves these FP64 runs by less
+than 4e-15, and FP32 rounding in the oracle itself the FP32 ones by less than 9e-7)."""
+import numpy as np
+import pytest
+
+from tests.helpers import rel_l2
+from tests.test_legacy2d import _gpu, _oracle, _synthetic
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,eps,scale", [
+    ("fp64", 1e-40, 1.0), ("fp64", 2e-39, 1.0), ("fp64", 1e-150, 1.0), ("fp64", 1e-7, 1e30), ("fp64", 1e-7, 1e70),
+    ("fp64", 1e40, 1e25), ("fp32", 1e-19, 1.0), ("fp32", 6e-20, 1.0), ("fp32", 1e-7, 1e9)])
+def test_legacy_scheme_at_the_ends_of_its_range(precision, eps, scale):
+    fx = _synthetic(2)
+    fx["eps"] = eps
+    for k in ("p0", "u0", "v0"):
+        fx[k] = fx[k] * scale
+    ir_o, f_o = _oracle(fx, fx["Nt"])
+    s = _gpu(fx, precision, fx["Nt"])
+    tol = 1e-10 if precision == "fp64" else 1e-5
+    got = [s.ir()] + list(s.fields())
+    s.close()
+    for a, b in zip(got, [ir_o] + list(f_o)):
+        assert np.isfinite(a).all()
+        assert rel_l2(a / scale, b / scale) < tol
