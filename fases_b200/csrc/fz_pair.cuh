@@ -106,16 +106,17 @@ __device__ __forceinline__ void weno_center(float2 qm2, float2 qm1, float2 q0, f
 // differences,
 //   3/4 beta_2 = a^2 - 11/4 a b + 5/2 b^2    3/4 beta_1 = b^2 - 5/4 b c + c^2
 //   3/4 beta_0 = 5/2 c^2 - 11/4 c d + d^2
-// (each at least 0.6 of its larger square, so rounding cannot make one negative; the 3/4 goes into
-// eps), and the weighted candidates 5 d_r (V_r - u_i), scaled so that most coefficients are 1:
+// (beta_1 is at least 0.6 of its larger square, the others at least 0.24 d^2 or a^2 and 0.6 c^2 or b^2, so
+// rounding cannot make one negative; the 3/4 goes into eps), and the weighted candidates 5 d_r (V_r - u_i), scaled so that most coefficients are 1:
 //   V-: c - d/4, c + b/2, (5 b - 2 a)/12      V+: -(5 c - 2 d)/12, -(b + c/2), -(b - a/4)
 // with the normaliser 5 sum d_r q_r: 37 operations a centre for both faces.
 // Nonlinear weights from the indicators B_r = 3/4 (beta_r + eps), up to a factor common to the three
 // (it cancels between the sums and their normalisers).
 //
 // Products of indicators leave the range of the type long before the indicators do (B lies between eps
-// and the square of the largest difference), so the 2D form scales by a power of two, which is exact and
-// leaves the bits of every other case alone: eps = 1e-40, or fields of 1e30, are as good as any.
+// and the square of the largest difference), so each form scales by a power of two, which is exact and
+// leaves the bits of every other case alone: a 2D solve with eps = 1e-40, or fields of 1e30, are as good
+// as any.
 
 // 2^-e for x = m 2^e, m in [1, 2), given x's upper word (FP64) or bits (FP32); x subnormal or zero: the
 // largest power of two (FP32: x finite)
@@ -126,8 +127,34 @@ __device__ __forceinline__ float pow2_inverse32(int bits) {
   return __int_as_float((254 << 23) - (bits & 0x7f800000));
 }
 
+// Reciprocal in 64 bits: the hardware's coarse seed (at least 20 bits) and one third-order
+// Householder step r (1 + e + e^2), e = 1 - x r, which leaves an error of e^3 < 2^-59 beside the
+// rounding of the last operation. For normal x below 2^1022 (no scaling, no special cases).
+__device__ __forceinline__ double drcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 struct WenoZ {  // 1 + tau / B_r, tau = |B_0 - B_2|
-  // In FP64 a reciprocal costs several FMA-pipe operations: the factors times B_0 B_1 B_2
+  // In FP64 a reciprocal costs several FMA-pipe operations: the factors times B_0 B_1 B_2. The weighted
+  // sums go up to B^3.5, so indicators from 2^256 on, differences above 1e38, are taken over the largest
+  // one's power of two, with a floor of 2^-256 (differences 1e-38 of the largest) in the place of the
+  // scaled eps. B_1 is at most 2.7 times the sum of the others. One test for both variables of a centre
+  // (190 x 150 x 140 cells: 1.5 % of a step; a test for each, which keeps their chains from being
+  // interleaved, 5 %; the products scaled without a test, 1.9 % and good to 1e94 only).
+  static constexpr int WIDE = (1023 + 256) << 20;
+  static __device__ __forceinline__ void range(double2& B0, double2& B1, double2& B2) {
+    const int x = max(__double2hiint(B0.x), __double2hiint(B2.x)), y = max(__double2hiint(B0.y), __double2hiint(B2.y));
+    if (max(x, y) >= WIDE) {
+      const double2 s = make_double2(pow2_inverse64(x), pow2_inverse64(y));
+      const double f = __hiloint2double((1023 - 256) << 20, 0);
+      B0 = pfma(B0, s, make_double2(f, f));
+      B1 = pfma(B1, s, make_double2(f, f));
+      B2 = pfma(B2, s, make_double2(f, f));
+    }
+  }
   __device__ __forceinline__ void operator()(double B0, double B1, double B2, double& w0, double& w1, double& w2) const {
     const double tau = fabs(B0 - B2);
     const double B12 = B1 * B2, B02 = B0 * B2, B01 = B0 * B1, B012 = B0 * B12;
@@ -154,6 +181,7 @@ struct WenoJS {
     w1 = pmul(q1, q1);
     w2 = pmul(q2, q2);
   }
+  static __device__ __forceinline__ void range(double2&, double2&, double2&) {}
   __device__ __forceinline__ void operator()(double B0, double B1, double B2, double& w0, double& w1, double& w2) const {
     const double P0 = B1 * B2, P1 = B0 * B2, P2 = B0 * B1;
     const double s = pow2_inverse64(max(max(__double2hiint(P0), __double2hiint(P1)), __double2hiint(P2)));
@@ -192,40 +220,21 @@ __device__ __forceinline__ void weno_sums(float2 qm2, float2 qm1, float2 q0, flo
   }
 }
 
-// Reciprocal in 64 bits: the hardware's coarse seed (at least 20 bits) and one third-order
-// Householder step r (1 + e + e^2), e = 1 - x r, which leaves an error of e^3 < 2^-59 beside the
-// rounding of the last operation. For normal x of moderate size (no scaling, no special cases).
-__device__ __forceinline__ double drcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
-// In FP64 the weights come without reciprocals (above) and both normalisers share one: 1 instead of 5
-// per variable (190 x 150 x 140 cells: a stage 0.175-0.183 ms instead of 0.265-0.272). B lies in
-// [eps, amplitude^2], so WenoZ's products (up to B^6) stay inside the double range for amplitudes below
-// 1e25.
+// In FP64 the weights come without reciprocals (above): 2 instead of 5 per variable (190 x 150 x 140 cells:
+// a stage 0.175-0.183 ms instead of 0.265-0.272; both normalisers on one reciprocal take the same time).
 template <int FACES, class W>
-__device__ __forceinline__ void weno_sums1(double qm2, double qm1, double q0, double qp1, double qp2, double eps,
+__device__ __forceinline__ void weno_sums1(double a, double b, double c, double d, double B0, double B1, double B2,
                                            W weights, double& Nm, double& Np, double& rSm, double& rSp) {
-  const double a = qm1 - qm2, b = q0 - qm1, c = qp1 - q0, d = qp2 - qp1;
-  const double bb = fma(b, b, eps);
-  const double B1 = fma(c, fma(b, -1.25, c), bb);
-  const double B2 = fma(a, fma(b, -2.75, a), fma(bb, 2.5, -1.5 * eps));
-  const double B0 = fma(d, fma(c, -2.75, d), fma(2.5 * c, c, eps));
   double w0, w1, w2;
   weights(B0, B1, B2, w0, w1, w2);
   const double t1 = 3.0 * w1;
-  const double Sm = fma(w0, 1.5, fma(w2, 0.5, t1)), Sp = fma(w0, 0.5, fma(w2, 1.5, t1));
-  const double r = drcp(Sm * Sp);
-  rSm = r * Sp;
-  rSp = r * Sm;
   if constexpr ((FACES & WENO_LO) != 0) {
+    rSm = drcp(fma(w0, 1.5, fma(w2, 0.5, t1)));
     const double e0 = fma(d, -0.25, c), e1 = fma(b, 0.5, c), e2 = fma(a, -1.0 / 6.0, b * (5.0 / 12.0));
     Nm = fma(w2, e2, fma(w1, e1, w0 * e0));
   }
   if constexpr ((FACES & WENO_HI) != 0) {
+    rSp = drcp(fma(w0, 0.5, fma(w2, 1.5, t1)));
     const double g0 = fma(d, -1.0 / 6.0, c * (5.0 / 12.0)), g1 = fma(c, 0.5, b), g2 = fma(a, -0.25, b);
     Np = fma(w2, g2, fma(w1, g1, w0 * g0));
   }
@@ -233,8 +242,15 @@ __device__ __forceinline__ void weno_sums1(double qm2, double qm1, double q0, do
 template <int FACES, class W>
 __device__ __forceinline__ void weno_sums(double2 qm2, double2 qm1, double2 q0, double2 qp1, double2 qp2, double eps,
                                           W weights, double2& Nm, double2& Np, double2& rSm, double2& rSp) {
-  weno_sums1<FACES>(qm2.x, qm1.x, q0.x, qp1.x, qp2.x, eps, weights, Nm.x, Np.x, rSm.x, rSp.x);
-  weno_sums1<FACES>(qm2.y, qm1.y, q0.y, qp1.y, qp2.y, eps, weights, Nm.y, Np.y, rSm.y, rSp.y);
+  auto K = [](double x) { return make_double2(x, x); };
+  const double2 a = psub(qm1, qm2), b = psub(q0, qm1), c = psub(qp1, q0), d = psub(qp2, qp1);
+  const double2 bb = pfma(b, b, K(eps));
+  double2 B1 = pfma(c, pfma(b, K(-1.25), c), bb);
+  double2 B2 = pfma(a, pfma(b, K(-2.75), a), pfma(bb, K(2.5), K(-1.5 * eps)));
+  double2 B0 = pfma(d, pfma(c, K(-2.75), d), pfma(pmul(c, K(2.5)), c, K(eps)));
+  W::range(B0, B1, B2);
+  weno_sums1<FACES>(a.x, b.x, c.x, d.x, B0.x, B1.x, B2.x, weights, Nm.x, Np.x, rSm.x, rSp.x);
+  weno_sums1<FACES>(a.y, b.y, c.y, d.y, B0.y, B1.y, B2.y, weights, Nm.y, Np.y, rSm.y, rSp.y);
 }
 
 // Outgoing characteristics of a centre, all the Godunov flux needs of it (functions3D.cuh:56-78 with

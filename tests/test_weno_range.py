@@ -7,7 +7,7 @@ than 4e-15, and FP32 rounding in the oracle itself the FP32 ones by less than 9e
 import numpy as np
 import pytest
 
-from tests.helpers import rel_l2
+from tests.helpers import rel_l2, run_gpu, run_oracle, small_room
 from tests.test_legacy2d import _gpu, _oracle, _synthetic
 
 
@@ -28,3 +28,22 @@ def test_legacy_scheme_at_the_ends_of_its_range(precision, eps, scale):
     for a, b in zip(got, [ir_o] + list(f_o)):
         assert np.isfinite(a).all()
         assert rel_l2(a / scale, b / scale) < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("depth", [0, 5])  # the direct and the marching kernel
+@pytest.mark.parametrize("scale", [1e20, 1e30, 1e70, 1e140])
+def test_fp64_stepper_with_large_fields(scale, depth):
+    cfg = small_room(seed=2, steps=60)
+    cfg["p0"] = cfg["p0"] * scale
+    cfg["sval"] = cfg["sval"] * scale
+    o = run_oracle(cfg)
+    s = run_gpu(cfg, "fp64", run=False)
+    if depth:
+        s.set_kz_chunk(depth)
+    s.run(cfg["steps"])
+    got = [s.ir()] + list(s.fields())
+    s.close()
+    for a, b in zip(got, [o.ir()[0]] + list(o.fields())):
+        assert np.isfinite(a).all()
+        assert rel_l2(a / scale, b / scale) < 1e-10
