@@ -43,6 +43,17 @@ __device__ __forceinline__ void rcp2(double2 a, double2 b, double2& ra, double2&
   rb = make_double2(x * a.x, y * a.y);
 }
 
+// The factor to apply to a centre's differences in FP64: one, or, where they reach 2^80, the power of two
+// that leaves the largest at 2^64, since the shared reciprocals take products of three indicators and of two
+// normalisers. A centre's derivatives do not depend on the scale of its differences (those below 1e-29
+// of the largest see an eps that is not scaled along). Multiplied without a branch: 2 % of the backward
+// pass of 78 x 66 x 54 cells, with a branch 9 % (spilled registers).
+__device__ __forceinline__ double narrowing(double a, double b, double c, double d) {
+  auto hi = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+  const int top = max(max(hi(a), hi(b)), max(hi(c), hi(d)));
+  return top >= (1023 + 80) << 20 ? pow2_inverse64(top) * 0x1p64 : 1.0;
+}
+
 // Reverse mode of one WENO-Z cell centre for a pair of variables (pressure and the velocity
 // component along the sweep): u[0..4] are the values at c-2 .. c+2; the centre gives V-(c+1/2)
 // (lam_m, its adjoint) and V+(c-1/2) (lam_p) from one set of smoothness indicators, as the
@@ -58,7 +69,14 @@ __device__ __forceinline__ void weno_centre_rev(const typename Pair<R>::T u[5], 
   auto K = [](double x) { return psplat<R>(R(x)); };
   constexpr double eps = 0.75e-10, k512 = 5.0 / 12.0, k16 = -1.0 / 6.0;
   // ---- forward (weno_sums)
-  const P a = psub(u[1], u[0]), b = psub(u[2], u[1]), c = psub(u[3], u[2]), d = psub(u[4], u[3]);
+  P a = psub(u[1], u[0]), b = psub(u[2], u[1]), c = psub(u[3], u[2]), d = psub(u[4], u[3]);
+  if constexpr (sizeof(R) == 8) {
+    const P s = pmk(narrowing(a.x, b.x, c.x, d.x), narrowing(a.y, b.y, c.y, d.y));
+    a = pmul(a, s);
+    b = pmul(b, s);
+    c = pmul(c, s);
+    d = pmul(d, s);
+  }
   const P t1 = pfma(b, K(-1.25), c), t2 = pfma(b, K(-2.75), a), t0 = pfma(c, K(-2.75), d);
   const P bb = pfma(b, b, K(eps));
   const P B1 = pfma(c, t1, bb);

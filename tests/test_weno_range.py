@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from tests.helpers import rel_l2, run_gpu, run_oracle, small_room
+from tests.test_adjoint import STEPS, _cfg, _solver
 from tests.test_legacy2d import _gpu, _oracle, _synthetic
 
 
@@ -47,3 +48,27 @@ def test_fp64_stepper_with_large_fields(scale, depth):
     for a, b in zip(got, [o.ir()[0]] + list(o.fields())):
         assert np.isfinite(a).all()
         assert rel_l2(a / scale, b / scale) < 1e-10
+
+
+@pytest.mark.gpu
+def test_fp64_gradient_scales_with_the_fields():
+    """Where eps does not count, the traces are homogeneous of degree one in the fields and J and its
+    gradient of degree two: with powers of two the same numbers but for the order of the sums (the probe
+    scatter's atomics) and the cells below 1e-29 of the largest difference."""
+    def gradient(scale):
+        cfg = _cfg()
+        cfg["p0"] = cfg["p0"] * scale
+        cfg["sval"] = cfg["sval"] * scale
+        s = _solver(cfg, "fp64")
+        target = scale * 1e-3 * np.random.default_rng(8).standard_normal((len(cfg["recs"]), STEPS))
+        g = s.misfit_gradient(target, segment_steps=16)
+        s.close()
+        return g
+
+    a, b = 2.0 ** 76, 2.0 ** 183  # 7.6e22 and 1.2e55
+    ga, gb = gradient(a), gradient(b)
+    assert abs(gb["J"] / b ** 2 / (ga["J"] / a ** 2) - 1.0) < 1e-12
+    for key in ("Rinf", "A", "zeta", "B", "C", "alpha", "beta"):
+        x, y = np.asarray(ga[key]) / a ** 2, np.asarray(gb[key]) / b ** 2
+        assert np.isfinite(y).all() and np.abs(x).max() > 0
+        assert rel_l2(y, x) < 1e-10, key
