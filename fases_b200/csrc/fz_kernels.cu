@@ -838,4 +838,28 @@ cudaError_t launch_receivers_group(const RecArgs<R>* args, int n, cudaStream_t s
 FZ_INSTANTIATE(float)
 FZ_INSTANTIATE(double)
 
+#ifdef FZ_WAIT_TEST
+namespace {
+__global__ void k_test_rcp(const double* x, double* y, int64_t n) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
+    y[q] = drcp(x[q]);
+}
+}  // namespace
+#endif
+
 }  // namespace fz
+
+#ifdef FZ_WAIT_TEST
+// Test build only: y[q] = drcp(x[q]), host arrays.
+extern "C" int fz_test_rcp(const double* x, double* y, int64_t n) {
+  double* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, (size_t)n * 16);
+  if (e == cudaSuccess) e = cudaMemcpy(d, x, (size_t)n * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    fz::k_test_rcp<<<64, 256>>>(d, d + n, n);
+    e = cudaMemcpy(y, d + n, (size_t)n * 8, cudaMemcpyDeviceToHost);
+  }
+  cudaFree(d);
+  return (int)e;
+}
+#endif
