@@ -368,21 +368,20 @@ int build_band(fz_handle* h) {
   return FZ_OK;
 }
 
-// Whether the room runs the direct stage kernel (fz_direct.cu): while its warps, 30 cells of a row
-// each, come to at most two waves of what the GPU holds (16 per SM). Measured, us a step, direct /
+// How far the room is up to the line of the direct stage kernel (fz_direct.cu), which it runs while its
+// warps, 30 cells of a row each, come to at most two waves of what the GPU holds (16 per SM). Measured, us a step, direct /
 // marching with chunks chosen for latency: 3D FP32 26 x 22 x 18 (396 warps) 15 / 27, 45 x 38 x 29 (2204)
 // 19 / 31, 58 x 46 x 40 (3680) 30 / 33, 71 x 53 x 47 (7473) 49 / 45, 64^3 69 / 45; FP64 19 / 31, 26 / 41,
 // 40 / 40, 70 / 60, 101 / 60. A planar room's direct kernel has no redundant centres to pay for, so it
 // goes a little further: FP32 256 x 256 (2304) 16 / 26, 500 x 400 (6800) 34 / 33, 800 x 800 104 / 60; FP64
 // 19 / 33, 44 / 50, 125 / 113.
-template <class R>
-bool use_direct(const fz_handle* h) {
+double direct_load(const fz_handle* h) {
 #ifdef FZ_WAIT_TEST
-  return false;  // this build is for the marching kernel's bounded waits
+  return 2.0;  // this build is for the marching kernel's bounded waits
 #else
   const int64_t tiles = (h->Nx - 2 * GHOST + fz::DIRECT_CELLS - 1) / fz::DIRECT_CELLS;
   const int64_t warps = tiles * (h->Ny - 2 * GHOST) * (h->prm.two_d ? 1 : h->Nz - 2 * GHOST) * h->nb;
-  return warps <= (int64_t)(h->prm.two_d ? 46 : 32) * h->nsm;
+  return (double)warps / ((h->prm.two_d ? 46.0 : 32.0) * h->nsm);
 #endif
 }
 
@@ -478,50 +477,11 @@ int finalize(fz_handle* h) {
   FZ_CUDA(h, fz::stage_occupancy<R>(&occ), "occupancy");
   occ = std::max(1, occ);
   h->stage_occ = occ;
-  const int ntx = (h->Nx - 2 * GHOST + fz::TX - 1) / fz::TX;
-  const int nty = (h->Ny - 2 * GHOST + fz::TY - 1) / fz::TY;
-  const int nzi = h->Nz - 2 * GHOST;
-  const int64_t slots = (int64_t)h->nsm * occ;
-  // Pick the z-chunk count that best fills whole waves of CTA slots, charging each chunk about
-  // 1.5 planes of start-up work (two extra z centres and the TMA ring fill).
-  int best = 1;
-  double best_eff = -1.0;
-  for (int nk = 1; nk <= std::max(1, nzi / 8); nk++) {
-    const int chunk = (nzi + nk - 1) / nk;
-    const int nk_eff = (nzi + chunk - 1) / chunk;
-    const int64_t items = (int64_t)ntx * nty * nk_eff * h->nb;
-    const int64_t waves = (items + slots - 1) / slots;
-    const double eff = ((double)items / (double)(waves * slots)) * ((double)chunk / (chunk + 1.5));
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = nk;
-    }
-  }
-  h->kz_heuristic = (nzi + best - 1) / best;
-  // A room that chunks of 8 planes spread over less than one wave: shallower chunks, by the launch's
-  // latency. In planes of a CTA alone on its SM, a launch takes c0 + sum over waves of (f chunk + c1),
-  // f = 1.45 where two CTAs share the SM; fitted to depths 1 .. 32 of rooms of 10^4 to 10^6 cells
-  // (71 x 53 x 47 FP32: depth 10, the wave model's choice, 84.6 us a step, depth 2 45.9; 64^3 84 -> 47;
-  // FP64 71 x 53 x 47 depth 4 114 -> 65). (Not in the wait-test build, whose hook names a plane of
-  // every chunk.)
-#ifndef FZ_WAIT_TEST
-  if ((int64_t)ntx * nty * h->nb * ((nzi + 7) / 8) <= slots) {
-    const double c0 = occ > 1 ? 1.2 : 2.0, c1 = occ > 1 ? 1.6 : 0.6;
-    double best_t = 1e300;
-    for (int c = 1; c <= nzi; c++) {
-      if (c < (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS) continue;
-      const int64_t items = (int64_t)ntx * nty * h->nb * ((nzi + c - 1) / c);
-      const int64_t full = items / slots, rest = items % slots;
-      const double shared = (occ > 1 ? 1.45 : 1.0) * c + c1;
-      const double t = c0 + full * shared + (rest == 0 ? 0.0 : rest <= h->nsm ? c + c1 : shared);
-      if (t < best_t - 1e-9) {
-        best_t = t;
-        h->kz_heuristic = c;
-      }
-    }
-  }
-#endif
-  h->direct_rule = use_direct<R>(h);
+  const fzi::StageTiles tiles = fzi::stage_tiles(h);
+  h->kz_heuristic = fzi::latency_depth({tiles}, h->nsm, occ);
+  if (h->kz_heuristic == 0) h->kz_heuristic = fzi::wave_depth(tiles, h->nsm, occ);
+  h->direct_load = direct_load(h);
+  h->direct_rule = h->direct_load <= 1.0;
   if (h->direct_rule && h->nB > 0 && !h->d_bidx) {
     // band index of every cell, from the band records
     std::vector<int4> rec((size_t)h->nB);
@@ -1041,7 +1001,47 @@ int bind_field_set(fz_handle* h, int set, void* const* f) {
 cudaError_t enqueue_stage_kernel(fz_handle* h, int st) {
   return h->fp64 ? ::enqueue_stage_kernel<double>(h, st) : ::enqueue_stage_kernel<float>(h, st);
 }
-int set_z_sizes(fz_handle* h, const std::vector<int>& sizes, bool direct) {
+namespace {
+dim3 plan_grid(const fz_handle* h, size_t chunks) {
+  const int ntx = (h->Nx - 2 * GHOST + fz::TX - 1) / fz::TX;
+  const int nty = (h->Ny - 2 * GHOST + fz::TY - 1) / fz::TY;
+  return dim3((unsigned)ntx, (unsigned)nty, (unsigned)(chunks * h->nb));
+}
+
+void set_plan(fz_handle* h, StagePlan p, bool z_auto) {
+  const bool same = p.zsizes == h->zsizes && p.grid.x == h->stage_grid.x && p.grid.y == h->stage_grid.y &&
+                    p.grid.z == h->stage_grid.z && p.direct == h->direct && z_auto == h->z_auto;
+  swap_plan(h, p);
+  h->z_auto = z_auto;
+  if (same) return;
+  h->launch_gen++;
+  for (auto& g : h->graph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+}
+}  // namespace
+
+void swap_plan(fz_handle* h, StagePlan& p) {
+  std::swap(h->zsizes, p.zsizes);
+  std::swap(h->stage_grid, p.grid);
+  std::swap(h->direct, p.direct);
+  h->zchunks = (int)h->zsizes.size();
+  h->kz_chunk = h->zsizes.empty() ? 0 : *std::max_element(h->zsizes.begin(), h->zsizes.end());
+}
+
+StagePlan uniform_plan(const fz_handle* h, int depth, bool direct) {
+  const int nzi = h->Nz - 2 * GHOST;
+  const int c = std::max(std::max(1, std::min(nzi, depth)), (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS);
+  StagePlan p;
+  for (int z = 0; z < nzi; z += c) p.zsizes.push_back(std::min(c, nzi - z));
+  p.grid = plan_grid(h, p.zsizes.size());
+  p.direct = direct;
+  return p;
+}
+
+int set_z_sizes(fz_handle* h, const std::vector<int>& sizes) {
   const int nzi = h->Nz - 2 * GHOST;
   int sum = 0;
   for (int c : sizes) {
@@ -1051,33 +1051,70 @@ int set_z_sizes(fz_handle* h, const std::vector<int>& sizes, bool direct) {
   if (sizes.empty() || (int)sizes.size() > fz::FZ_MAX_ZCHUNKS || sum != nzi)
     return set_error(h, FZ_EINVAL, "z chunks must cover the interior planes in at most " +
                                        std::to_string(fz::FZ_MAX_ZCHUNKS) + " pieces");
-  const int ntx = (h->Nx - 2 * GHOST + fz::TX - 1) / fz::TX;
-  const int nty = (h->Ny - 2 * GHOST + fz::TY - 1) / fz::TY;
-  const dim3 grid((unsigned)ntx, (unsigned)nty, (unsigned)(sizes.size() * h->nb));
-  const bool same = sizes == h->zsizes && grid.x == h->stage_grid.x && grid.y == h->stage_grid.y &&
-                    grid.z == h->stage_grid.z && h->direct == direct;
-  h->direct = direct;
-  h->zsizes = sizes;
-  h->zchunks = (int)sizes.size();
-  h->kz_chunk = *std::max_element(sizes.begin(), sizes.end());
-  h->stage_grid = grid;
-  if (same) return FZ_OK;
-  h->launch_gen++;
-  for (auto& g : h->graph)
-    if (g) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
+  set_plan(h, StagePlan{sizes, plan_grid(h, sizes.size()), false}, false);
   return FZ_OK;
 }
 
 void set_kz_chunk(fz_handle* h, int kz_chunk) {
-  const int nzi = h->Nz - 2 * GHOST;
-  int c = std::max(1, std::min(nzi, kz_chunk > 0 ? kz_chunk : h->kz_heuristic));
-  c = std::max(c, (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS);
-  std::vector<int> sizes;
-  for (int z = 0; z < nzi; z += c) sizes.push_back(std::min(c, nzi - z));
-  set_z_sizes(h, sizes, kz_chunk <= 0 && h->direct_rule);
+  const bool z_auto = kz_chunk <= 0;
+  set_plan(h, uniform_plan(h, z_auto ? h->kz_heuristic : kz_chunk, z_auto && h->direct_rule), z_auto);
+}
+
+StageTiles stage_tiles(const fz_handle* h) {
+  const dim3 one = plan_grid(h, 1);
+  return {(int64_t)one.x * one.y * one.z, h->Nz - 2 * GHOST};
+}
+
+int wave_depth(const StageTiles& room, int nsm, int occ) {
+  // the z-chunk count that best fills whole waves of CTA slots, charging each chunk about 1.5 planes of
+  // start-up work (two extra z centres and the TMA ring fill)
+  const int64_t slots = (int64_t)nsm * occ;
+  int depth = room.planes;
+  double best_eff = -1.0;
+  for (int nk = 1; nk <= std::max(1, room.planes / 8); nk++) {
+    const int chunk = (room.planes + nk - 1) / nk;
+    const int64_t items = room.columns * ((room.planes + chunk - 1) / chunk);
+    const int64_t waves = (items + slots - 1) / slots;
+    const double eff = ((double)items / (double)(waves * slots)) * ((double)chunk / (chunk + 1.5));
+    if (eff > best_eff + 1e-9) {
+      best_eff = eff;
+      depth = chunk;
+    }
+  }
+  return depth;
+}
+
+int latency_depth(const std::vector<StageTiles>& rooms, int nsm, int occ) {
+#ifdef FZ_WAIT_TEST
+  return 0;  // this build's hook names a plane of every chunk
+#else
+  // In planes of a CTA alone on its SM, a launch takes c0 + sum over waves of (f chunk + c1), f = 1.45 where
+  // two CTAs share the SM; fitted to depths 1 .. 32 of rooms of 10^4 to 10^6 cells (71 x 53 x 47 FP32: depth
+  // 10, the wave model's choice, 84.6 us a step, depth 2 45.9; 64^3 84 -> 47; FP64 71 x 53 x 47 depth 4
+  // 114 -> 65).
+  const int64_t slots = (int64_t)nsm * occ;
+  int nzi = 1;
+  for (const StageTiles& r : rooms) nzi = std::max(nzi, r.planes);
+  auto ctas = [&](int c) {
+    int64_t n = 0;
+    for (const StageTiles& r : rooms) n += r.columns * ((r.planes + c - 1) / c);
+    return n;
+  };
+  if (ctas(8) > slots) return 0;
+  const double c0 = occ > 1 ? 1.2 : 2.0, c1 = occ > 1 ? 1.6 : 0.6;
+  int depth = nzi;
+  double best_t = 1e300;
+  for (int c = (nzi + fz::FZ_MAX_ZCHUNKS - 1) / fz::FZ_MAX_ZCHUNKS; c <= nzi; c++) {
+    const int64_t items = ctas(c), full = items / slots, rest = items % slots;
+    const double shared = (occ > 1 ? 1.45 : 1.0) * c + c1;
+    const double t = c0 + full * shared + (rest == 0 ? 0.0 : rest <= nsm ? c + c1 : shared);
+    if (t < best_t - 1e-9) {
+      best_t = t;
+      depth = c;
+    }
+  }
+  return depth;
+#endif
 }
 
 std::vector<int> guided_z_sizes(fz_handle* h, int depth) {

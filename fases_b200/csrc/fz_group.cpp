@@ -58,6 +58,9 @@ struct fz_group {
   // shared launches run as `nbranch` concurrent branches (streams), each over a set of members of
   // about equal cells, so one branch's band and receiver launches overlap another's stage launch
   int nbranch = 1;
+  // stage launches of the members whose depth was not set: chosen for all of them side by side, where the
+  // member's own choice is for its room alone
+  std::vector<fzi::StagePlan> plan;
   std::vector<int> branch_of;  // branch of each member
   std::vector<cudaStream_t> bstream;
   std::vector<cudaEvent_t> bjoin;
@@ -87,6 +90,42 @@ int order_after(fz_group* g, bool members_wait_for_group) {
     }
   }
   return FZ_OK;
+}
+
+// Launches made while this lives take the group's plans (the members' own return with it).
+struct WithPlans {
+  fz_group* g;
+  explicit WithPlans(fz_group* g_) : g(g_) { exchange(); }
+  ~WithPlans() { exchange(); }
+  WithPlans(const WithPlans&) = delete;
+  void exchange() {
+    for (size_t q = 0; q < g->m.size(); q++)
+      if (g->m[q]->z_auto) fzi::swap_plan(g->m[q], g->plan[q]);
+  }
+};
+
+// The plans for all members side by side. Chunks by latency while those of 8 planes of all rooms together are
+// less than one wave, else each room's wave-filling depth. Members' own launches use the direct kernel while
+// all rooms together stay below twice a room's line (their launches overlap only in part). Untuned, us a step
+// of all rooms, shared launches / members' own, with the choices of the rooms alone -> with these: FP32
+// sixteen 48^3 360 / 529 -> 235 / 230, 32 rooms of 20 to 50 cells an edge 386 / 527 -> 248 / 259, six of 64^3
+// 199 / 180 -> 183 / 157; FP64 524 / 733 -> 422 / 409, 629 / 725 -> 451 / 445, 305 / 292 -> 298 / 271. The line,
+// members' launches direct / marching, by the rooms' load: FP32 1.35 37 / 46, 2.0 53 / 55, 2.3 66 / 64, 2.7
+// 70 / 65, 4.1 113 / 81; FP64 1.35 51 / 64, 2.0 75 / 74, 2.3 100 / 97, 4.1 178 / 122.
+void make_plans(fz_group* g) {
+  std::vector<fzi::StageTiles> rooms;
+  double load = 0.0;
+  for (const fz_handle* h : g->m) {
+    rooms.push_back(fzi::stage_tiles(h));
+    load += h->direct_load;
+  }
+  g->plan.clear();
+  for (size_t q = 0; q < g->m.size(); q++) {
+    const fz_handle* h = g->m[q];
+    int depth = fzi::latency_depth(rooms, h->nsm, h->stage_occ);
+    if (depth == 0) depth = fzi::wave_depth(rooms[q], h->nsm, h->stage_occ);
+    g->plan.push_back(fzi::uniform_plan(h, depth, h->direct_rule && load <= 2.0));
+  }
 }
 
 std::vector<int> parity_key(const fz_group* g) {
@@ -263,6 +302,7 @@ int flat_tables(fz_group* g, const std::vector<int>& key) {
 int ensure_flat_tables(fz_group* g) {
   int rc = ensure_branch_streams(g);
   if (rc != FZ_OK) return rc;
+  const WithPlans plans(g);
   for (int flip = 0; flip < 2; flip++) {
     rc = g->fp64 ? flat_tables<double>(g, parity_key(g)) : flat_tables<float>(g, parity_key(g));
     for (fz_handle* h : g->m) fzi::rotate(h);
@@ -324,6 +364,7 @@ cudaError_t flat_trial_kernels(fz_group* g, const FlatTables& t, int n) {
 
 // The same trial for each member's own launches, side by side on the members' streams.
 cudaError_t member_trial_kernels(fz_group* g, int n) {
+  const WithPlans plans(g);
   cudaError_t e = cudaEventRecord(g->fork, g->stream);
   for (size_t q = 0; q < g->m.size() && e == cudaSuccess; q++) {
     fz_handle* h = g->m[q];
@@ -369,6 +410,7 @@ cudaError_t flat_enqueue(fz_group* g, int nsteps) {
 }
 
 int capture(fz_group* g, cudaGraphExec_t* out) {
+  const WithPlans plans(g);
   cudaGraph_t graph = nullptr;
   FZ_GCUDA(g, cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
   cudaError_t e = cudaEventRecord(g->fork, g->stream);
@@ -440,6 +482,7 @@ int fz_group_create(fz_handle* const* members, int32_t n, fz_group** out) {
   g->flat_ok = n <= fz::FZ_MAX_GROUP;
   for (fz_handle* h : g->m)
     if (h->fp64 != g->fp64 || h->prm.two_d || h->sl_on) g->flat_ok = false;
+  make_plans(g);
   set_mode(g, 0);
   g->bstream.push_back(nullptr);  // branch 0 runs on the group stream
   g->bjoin.push_back(nullptr);
@@ -530,6 +573,7 @@ int fz_group_run(fz_group* g, int64_t nsteps) {
     rc = order_after(g, true);  // later work on a member (fz_sync, fz_get_ir, fz_run) follows
     if (rc != FZ_OK) return rc;
   }
+  const WithPlans plans(g);
   for (; done < nsteps; done++)
     for (fz_handle* h : g->m) {
       const cudaError_t e = fzi::enqueue(h);
@@ -544,7 +588,7 @@ int fz_group_autotune(fz_group* g, int32_t reps, int32_t* kz_chunk, double* ms_p
   int rc = fz_group_sync(g, 0);
   if (rc != FZ_OK) return rc;
   cudaSetDevice(g->device);
-  // one depth for every member (clamped to each room's planes), or 0: each member's own heuristic
+  // one depth for every member (clamped to each room's planes), or 0: the group's own choice
   int nzmax = 1;
   for (fz_handle* h : g->m) nzmax = std::max(nzmax, h->Nz - 2 * fz::GHOST);
   std::vector<fzi::ZPlan> cand{{0, 0}};

@@ -124,13 +124,15 @@ struct fz_handle {
   int seq = 0;
   bool finalized = false;
   int kz_chunk = 0;       // largest z chunk of the stage kernels
-  int kz_heuristic = 0;  // the wave-filling choice of prepare (fz_set_kz_chunk(h, 0) returns to it)
+  int kz_heuristic = 0;  // the choice of prepare for the room alone (fz_set_kz_chunk(h, 0) returns to it)
+  bool z_auto = true;    // that choice is in force: no depth or schedule was set
   int zchunks = 1;       // z chunks per member
   std::vector<int> zsizes;  // their lengths in planes (sum = interior planes), longest first
   int stage_occ = 1;        // stage-kernel CTAs per SM
-  // the direct stage kernel of small rooms (fz_direct.cu): whether the room's size calls for it,
-  // whether the launches use it now (an explicit tile depth or schedule selects the marching kernel),
-  // and its band index per cell
+  // the direct stage kernel of small rooms (fz_direct.cu): the room's warps over the most that call for
+  // it, whether they do, whether the launches use it now (an explicit tile depth or schedule selects the
+  // marching kernel), and its band index per cell
+  double direct_load = 0.0;
   bool direct_rule = false, direct = false;
   int32_t* d_bidx = nullptr;
   dim3 stage_grid;
@@ -185,9 +187,28 @@ cudaError_t enqueue_stage_kernel(fz_handle* h, int st);
 // handle's captured graphs
 void set_kz_chunk(fz_handle* h, int kz_chunk);
 // z chunks of any lengths (summing to the interior planes, at most FZ_MAX_ZCHUNKS) of the marching
-// stage kernel, or (direct) the direct kernel with those chunks kept for the shared launches of a
-// group; drops graphs
-int set_z_sizes(fz_handle* h, const std::vector<int>& sizes, bool direct = false);
+// stage kernel; drops graphs
+int set_z_sizes(fz_handle* h, const std::vector<int>& sizes);
+// Stage CTAs of a room one plane deep, and its interior planes.
+struct StageTiles {
+  int64_t columns;
+  int planes;
+};
+StageTiles stage_tiles(const fz_handle* h);
+// Tile depths, occ CTAs an SM: that which best fills whole waves with one room; that of the least latency for
+// rooms whose stage kernels run side by side, where their 8-plane chunks are less than one wave (else 0).
+int wave_depth(const StageTiles& room, int nsm, int occ);
+int latency_depth(const std::vector<StageTiles>& rooms, int nsm, int occ);
+// What a handle's stage launches take from its z chunks and kernel choice.
+struct StagePlan {
+  std::vector<int> zsizes;
+  dim3 grid;
+  bool direct;
+};
+StagePlan uniform_plan(const fz_handle* h, int depth, bool direct);
+// exchanges the handle's plan and p, leaving its graphs and tables alone: for launches made with p
+// before it is exchanged back
+void swap_plan(fz_handle* h, StagePlan& p);
 // a guided schedule: chunks of `depth` planes, then about one wave of CTAs at depth/2 and one at
 // depth/4, so the last waves are short
 std::vector<int> guided_z_sizes(fz_handle* h, int depth);

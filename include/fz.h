@@ -255,7 +255,9 @@ int fz_group_set_branches(fz_group* g, int32_t branches);
  * (the call does not advance the solve). kz_chunk gets the chosen (longest) chunk, ms_per_step the
  * stage kernels' time per step; fz_get_z_schedule lists the chunks. fz_group_autotune does the
  * same for all members at once, timing their kernels side by side with one uniform depth for every
- * member (clamped to each room; 0 = each member's heuristic). Results do not depend on the depth (each CTA recomputes its boundary centres).
+ * member (clamped to each room; 0 = the group's own choice). Results do not depend on the depth (each CTA
+ * recomputes its boundary centres). Members whose depth was not set run in a group with launches chosen for
+ * all its rooms side by side, and with their own again outside it.
  * Small rooms run a kernel without chunks (stage and band in one launch) unless a depth or schedule is
  * set; where that applies the trials time stage and band kernels and it is one of the candidates; when it
  * wins, kz_chunk is the heuristic depth, and another handle gets the same kernel by depth 0.

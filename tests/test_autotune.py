@@ -95,3 +95,37 @@ def test_tuning_batched_and_grouped_solves():
             assert np.array_equal(s.ir(), r)
     for s in members:
         s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("branches", [0, -1])
+def test_untuned_group_chooses_for_all_rooms_together(branches):
+    """Sixteen rooms of 48^3 fill the GPU together, so the launches that suit one of them alone (one-plane
+    chunks, the direct kernel) are not theirs: an untuned group takes at most a quarter longer than one
+    whose members are set to eight-plane chunks (with the rooms' own choices it took 1.5 and 2.2 times as
+    long), and gives the same traces. Alone, a member runs as it would without the group."""
+    from fases_b200 import Group
+    cfgs = [small_room(seed=50 + q, room=(48, 48, 48), steps=200) for q in range(16)]
+
+    def step_us(depth):
+        members = [_solver(c, steps=cfgs[0]["steps"]) for c in cfgs]
+        own = [s.z_schedule() for s in members]
+        if depth:
+            for s in members:
+                s.set_kz_chunk(depth)
+        with Group(members) as g:
+            g.set_branches(branches)
+            g.run(40)
+            us = min(g.run_timed(40) for _ in range(4)) / 40 * 1e3
+        ir = [s.ir() for s in members]
+        if not depth:
+            assert [s.z_schedule() for s in members] == own
+        for s in members:
+            s.close()
+        return us, ir
+
+    default, ir = step_us(0)
+    deep, ir_deep = step_us(8)
+    assert default <= 1.25 * deep, (default, deep)
+    for a, b in zip(ir, ir_deep):
+        assert np.array_equal(a, b)
