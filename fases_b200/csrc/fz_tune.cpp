@@ -8,10 +8,12 @@
 // by side, as the group's graphs run them. The reference launches fixed TP(32,4,4) blocks
 // (3D-solver/core/main3D.cu:1280-1306) and has no tuner.
 //
-// The trials launch the three stage kernels only. Their outputs land in the field sets U1 and U2,
-// whose updated cells the next real step rewrites before reading; the cPML psi tiles (advanced by
-// stage 2) and the output cells of sources in skipped cells (which accumulate) are saved before
-// and restored after, so the solve continues exactly as it would have.
+// The trials launch the three stage kernels only, or, for groups and for rooms small enough for the
+// direct kernel, which includes the band, stages and bands. Their outputs land in the field sets U1 and U2,
+// whose updated cells the next real step rewrites before reading, and in the ADE sets that it writes
+// before it reads them; the cPML psi tiles (advanced by stage 2) and the output cells of sources in
+// skipped cells (which accumulate) are saved before and restored after, so the solve continues exactly as
+// it would have. Trials are not entered into a profile.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -77,6 +79,22 @@ int restore_state(fz_handle* h, Saved& sv) {
   return FZ_OK;
 }
 
+// Per-launch timers off while this lives.
+struct Unprofiled {
+  std::vector<fz_handle*> on;
+  explicit Unprofiled(const std::vector<fz_handle*>& hs) {
+    for (fz_handle* h : hs)
+      if (h->profiling) {
+        on.push_back(h);
+        h->profiling = false;
+      }
+  }
+  ~Unprofiled() {
+    for (fz_handle* h : on) h->profiling = true;
+  }
+  Unprofiled(const Unprofiled&) = delete;
+};
+
 }  // namespace
 
 namespace fzi {
@@ -128,6 +146,7 @@ int tune(const std::vector<fz_handle*>& hs, cudaStream_t ts, const std::vector<Z
     const int rc = fz_sync(h, 0);
     if (rc != FZ_OK) return rc;
   }
+  const Unprofiled unprofiled(hs);
   cudaSetDevice(hs[0]->device);
   std::vector<Saved> saved(hs.size());
   for (size_t q = 0; q < hs.size(); q++) {

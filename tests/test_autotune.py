@@ -129,3 +129,17 @@ def test_untuned_group_chooses_for_all_rooms_together(branches):
     assert default <= 1.25 * deep, (default, deep)
     for a, b in zip(ir, ir_deep):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room", [(26, 22, 18), (71, 53, 47)])
+def test_tuning_is_not_entered_into_a_profile(room):
+    s = _solver(small_room(seed=7, room=room, steps=40))
+    s.profile(True)
+    s.run(1)
+    s.profile_read()
+    s.autotune(reps=2)
+    assert all(n == 0 for _, n in s.profile_read().values())
+    s.run(1)
+    assert s.profile_read()["stage0"][1] == 1
+    s.close()
