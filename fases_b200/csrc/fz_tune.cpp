@@ -108,6 +108,7 @@ int apply_z_plan(fz_handle* h, const ZPlan& p) {
 std::vector<ZPlan> kz_candidates(fz_handle* h) {
   const int nzi = h->Nz - 2 * GHOST;
   std::vector<ZPlan> out{{0, 0}};
+  if (h->direct_rule) out.push_back({h->kz_heuristic, 0});  // {0, 0} is the direct kernel then
   if (nzi <= 1) return out;
   // every distinct depth ceil(nzi / nk) of at least 2 planes, ranked by the heuristic's model
   const int occ = std::max(1, h->stage_occ);
@@ -128,7 +129,8 @@ std::vector<ZPlan> kz_candidates(fz_handle* h) {
   std::sort(ranked.begin(), ranked.end(), [](const std::pair<double, int>& a, const std::pair<double, int>& b) {
     return a.first > b.first || (a.first == b.first && a.second > b.second);
   });
-  for (size_t q = 0; q < ranked.size() && out.size() < 9; q++)
+  const size_t most = out.size() + 8;
+  for (size_t q = 0; q < ranked.size() && out.size() < most; q++)
     if (ranked[q].second != h->kz_heuristic) out.push_back({ranked[q].second, 0});
   // guided schedules: long chunks first, short ones for the last waves (single rooms; a batch's
   // members run one after another in the grid, so its tail is one member's)
@@ -250,6 +252,8 @@ int fz_set_kz_chunk(fz_handle* h, int32_t kz_chunk) {
   if (rc != FZ_OK) return rc;
   rc = fz_sync(h, 0);
   if (rc != FZ_OK) return rc;
+  // the depth that fz_autotune gives where the direct kernel won
+  if (h->direct_rule && kz_chunk == h->kz_heuristic) kz_chunk = 0;
   fzi::set_kz_chunk(h, kz_chunk);
   return FZ_OK;
 }
@@ -273,7 +277,12 @@ int fz_set_z_schedule(fz_handle* h, const int32_t* sizes, int32_t n) {
   if (rc != FZ_OK) return rc;
   rc = fz_sync(h, 0);
   if (rc != FZ_OK) return rc;
-  return fzi::set_z_sizes(h, std::vector<int>(sizes, sizes + n));
+  const std::vector<int> z(sizes, sizes + n);
+  if (h->direct_rule && z == fzi::uniform_plan(h, h->kz_heuristic, true).zsizes) {  // as fz_set_kz_chunk
+    fzi::set_kz_chunk(h, 0);
+    return FZ_OK;
+  }
+  return fzi::set_z_sizes(h, z);
 }
 
 int fz_get_kz_chunk(fz_handle* h, int32_t* kz_chunk, int32_t* heuristic) {

@@ -153,7 +153,9 @@ def main(argv=None):
     s, nt = Solver.from_project(scene, config, src, rec, precision=precision)
     if nt >= 200 and "--no-autotune" not in argv:
         depth, _ = s.autotune()  # a few stage launches; pays for itself on runs of this length
-        print(f"[OK] stage tile depth {depth} planes (autotuned)", flush=True)
+        own = depth == s.kz_chunk()[1]  # the heuristic depth, or a small room's kernel without chunks
+        print(f"[OK] stage launches {'as the heuristic has them' if own else f'tile depth {depth} planes'} (autotuned)",
+              flush=True)
     print(f"[OK] Will now start {nt} iterations", flush=True)
     t0 = time.perf_counter()
     s.run_progress(nt, lambda done, total: print("%d%%" % int(100.0 * done / total + 0.5), flush=True), 5)

@@ -214,8 +214,8 @@ class Solver:
         return k.value, ms.value
 
     def set_kz_chunk(self, depth):
-        """Tile depth of the stage kernels (0 = the heuristic: chunks that fill whole waves, or for small
-        rooms the kernel without chunks), e.g. from a cache."""
+        """Tile depth of the stage kernels (0, or the heuristic depth itself = the heuristic: chunks that
+        fill whole waves, or for small rooms the kernel without chunks), e.g. from a cache."""
         self._chk(lib().fz_set_kz_chunk(self._h, int(depth)))
 
     def z_schedule(self):

@@ -258,13 +258,15 @@ int fz_group_set_branches(fz_group* g, int32_t branches);
  * member (clamped to each room; 0 = the group's own choice). Results do not depend on the depth (each CTA
  * recomputes its boundary centres). Members whose depth was not set run in a group with launches chosen for
  * all its rooms side by side, and with their own again outside it.
- * Small rooms run a kernel without chunks (stage and band in one launch) unless a depth or schedule is
- * set; where that applies the trials time stage and band kernels and it is one of the candidates; when it
- * wins, kz_chunk is the heuristic depth, and another handle gets the same kernel by depth 0.
+ * Small rooms run a kernel without chunks (stage and band in one launch) unless another depth or schedule
+ * than the heuristic one is set; where that applies the trials time stage and band kernels and both it and the
+ * chunked kernel at the heuristic depth are candidates; when it wins, kz_chunk is the heuristic depth, which
+ * selects it again (as depth 0 does, and the heuristic schedule).
  * The reference launches fixed TP(32,4,4) blocks (main3D.cu:1280-1306). */
 int fz_autotune(fz_handle* h, int32_t reps, int32_t* kz_chunk, double* ms_per_step);
 int fz_group_autotune(fz_group* g, int32_t reps, int32_t* kz_chunk, double* ms_per_step);
-/* Sets the depth directly (0 = the heuristic), e.g. from a cache of earlier tuning results. */
+/* Sets the depth directly (0 = the heuristic, or that depth itself), e.g. from a cache of earlier tuning
+ * results. */
 int fz_set_kz_chunk(fz_handle* h, int32_t kz_chunk);
 int fz_get_kz_chunk(fz_handle* h, int32_t* kz_chunk, int32_t* heuristic);
 /* The z chunks the stage kernels use now (lengths in planes, longest first; the tuner may pick a

@@ -131,6 +131,35 @@ def test_untuned_group_chooses_for_all_rooms_together(branches):
         assert np.array_equal(a, b)
 
 
+def _band_launches(s):
+    s.profile(True)
+    s.run(2)
+    n = s.profile_read()["band"][1]
+    s.profile(False)
+    return n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_tuned_launches_come_back_from_the_depth_and_the_schedule(precision):
+    """In a room this small the direct kernel (no band launches) wins by far; the depth that the tuner
+    returns, and the schedule, select it again on another handle, and any other depth does not."""
+    cfg = small_room(seed=7, steps=40)
+    s = _solver(cfg, precision)
+    depth, _ = s.autotune(reps=3)
+    sched = s.z_schedule()
+    assert _band_launches(s) == 0
+    other = 4 if depth != 4 else 5
+    for select, launches in ((lambda x: x.set_kz_chunk(depth), 0), (lambda x: x.set_z_schedule(sched), 0),
+                             (lambda x: x.set_kz_chunk(0), 0), (lambda x: x.set_kz_chunk(other), 6)):
+        t = _solver(cfg, precision)
+        t.set_kz_chunk(other)
+        select(t)
+        assert _band_launches(t) == launches
+        t.close()
+    s.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("room", [(26, 22, 18), (71, 53, 47)])
 def test_tuning_is_not_entered_into_a_profile(room):
