@@ -369,19 +369,21 @@ int build_band(fz_handle* h) {
 }
 
 // How far the room is up to the line of the direct stage kernel (fz_direct.cu), which it runs while its
-// warps, 30 cells of a row each, come to at most two waves of what the GPU holds (16 per SM). Measured, us a step, direct /
-// marching with chunks chosen for latency: 3D FP32 26 x 22 x 18 (396 warps) 15 / 27, 45 x 38 x 29 (2204)
-// 19 / 31, 58 x 46 x 40 (3680) 30 / 33, 71 x 53 x 47 (7473) 49 / 45, 64^3 69 / 45; FP64 19 / 31, 26 / 41,
-// 40 / 40, 70 / 60, 101 / 60. A planar room's direct kernel has no redundant centres to pay for, so it
-// goes a little further: FP32 256 x 256 (2304) 16 / 26, 500 x 400 (6800) 34 / 33, 800 x 800 104 / 60; FP64
-// 19 / 33, 44 / 50, 125 / 113.
+// warps, 30 cells of a row each, come to at most two waves of what the GPU holds (16 per SM). us a step,
+// direct / marching at its best depth, by warps an SM: 3D FP32 6 16 / 27, 15 18 / 32, 25 30 / 33, 29 32 / 33, 31.6
+// (60 x 52 x 45) 32 / 39, 50 (71 x 53 x 47) 49 / 45; FP64 15 25 / 40, 25 40 / 40, 29 (58 x 46 x 46) 43 / 40, 30 (60 x
+// 50 x 44) 44 / 49, 31 (29 x 70 x 66) 46 / 52, 50 70 / 60: between 25 and 32 the ragged tiles of the marching kernel
+// decide. A planar room's direct kernel has no redundant centres to pay for, but its marching kernel
+// launches once for all planes: FP32 16 (256 x 256) 16 / 26, 28 (350 x 350) 23 / 28, 30.4 (90 x 1500) 29 / 28, 36 33 /
+// 32, 46 (500 x 400) 34.5 / 33.2; FP64 28 28 / 36, 46 39 / 47, 145 (800 x 800) 125 / 113.
 double direct_load(const fz_handle* h) {
 #ifdef FZ_WAIT_TEST
   return 2.0;  // this build is for the marching kernel's bounded waits
 #else
   const int64_t tiles = (h->Nx - 2 * GHOST + fz::DIRECT_CELLS - 1) / fz::DIRECT_CELLS;
   const int64_t warps = tiles * (h->Ny - 2 * GHOST) * (h->prm.two_d ? 1 : h->Nz - 2 * GHOST) * h->nb;
-  return (double)warps / ((h->prm.two_d ? 46.0 : 32.0) * h->nsm);
+  const double line = !h->prm.two_d ? 32.0 : h->fp64 ? 46.0 : 30.0;
+  return (double)warps / (line * h->nsm);
 #endif
 }
 

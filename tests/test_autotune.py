@@ -172,3 +172,20 @@ def test_tuning_is_not_entered_into_a_profile(room):
     s.run(1)
     assert s.profile_read()["stage0"][1] == 1
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room,precision,direct", [((256, 256), "fp32", True), ((500, 400), "fp32", False),
+                                                   ((500, 400), "fp64", True), ((640, 500), "fp64", False)])
+def test_planar_rooms_take_the_faster_kernel(room, precision, direct):
+    """Either side of the line between the direct and the marching kernel, which lies lower in FP32 (500 x 400:
+    34.5 us a step direct, 33.2 marching; FP64 39 and 47). The direct kernel launches no bands."""
+    from fases_b200 import Solver, params, scenes
+    from fases_b200 import materials as mats
+    sc = scenes.box_room_2d(room, 0.05)
+    s = Solver(params(h=0.05, precision=precision, two_d=True))
+    s.load_geometry(sc.S, sc.oid)
+    m = mats.pack([mats.rigid(0.9)] * 4)
+    s.set_materials(m["Rinf"], m["A"], m["zeta"], m["B"], m["Cc"], m["alpha"], m["beta"])
+    assert _band_launches(s) == (0 if direct else 6)
+    s.close()
