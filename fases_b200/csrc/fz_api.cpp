@@ -414,7 +414,6 @@ int finalize(fz_handle* h) {
   FZ_CUDA(h, cudaMemcpy(h->d_mat, packed.data(), packed.size() * 8, cudaMemcpyHostToDevice), "materials H2D");
   // ADE states (3 rotating sets, main3D.cu:683-709), zeroed
   if (h->nB > 0) {
-    FZ_CUDA(h, cudaMalloc(&h->d_wst, (size_t)h->nB * 2 * 8), "cudaMalloc(ADE)");
     const size_t nk = (size_t)h->nB * h->K, nl = (size_t)h->nB * h->L;
     for (int s = 0; s < 3; s++) {
       FZ_CUDA(h, cudaMalloc(&h->d_ade[s][0], nk * 8), "cudaMalloc(ADE)");
@@ -484,20 +483,17 @@ int finalize(fz_handle* h) {
   if (h->kz_heuristic == 0) h->kz_heuristic = fzi::wave_depth(tiles, h->nsm, occ);
   h->direct_load = direct_load(h);
   h->direct_rule = h->direct_load <= 1.0;
+  // copies from pageable memory may still be on their way when cudaMemcpy returns, and the handle's stream
+  // does not wait for the default stream
+  FZ_CUDA(h, cudaStreamSynchronize(cudaStreamLegacy), "set-up copies");
   if (h->direct_rule && h->nB > 0 && !h->d_bidx) {
-    // band index of every cell, from the band records
-    std::vector<int4> rec((size_t)h->nB);
-    FZ_CUDA(h, cudaMemcpy(rec.data(), h->d_brec, rec.size() * sizeof(int4), cudaMemcpyDeviceToHost), "band D2H");
-    std::vector<int32_t> bidx((size_t)(h->ncell_dev * h->nb), -1);
-    for (size_t b = 0; b < rec.size(); b++)
-      bidx[(size_t)(((uint64_t)(uint32_t)rec[b].y << 32) | (uint32_t)rec[b].x)] = (int32_t)b;
-    FZ_CUDA(h, cudaMalloc(&h->d_bidx, bidx.size() * sizeof(int32_t)), "cudaMalloc(band index)");
-    FZ_CUDA(h, cudaMemcpy(h->d_bidx, bidx.data(), bidx.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
-            "band index H2D");
+    const size_t n = (size_t)(h->ncell_dev * h->nb);
+    FZ_CUDA(h, cudaMalloc(&h->d_bidx, n * sizeof(int32_t)), "cudaMalloc(band index)");
+    FZ_CUDA(h, fz::launch_band_index(h->d_brec, h->nB, h->d_bidx, n, h->stream), "band index");
   }
-  h->finalized = true;
-  fzi::set_kz_chunk(h, h->kz_chunk > 0 ? h->kz_chunk : 0);
-  return FZ_OK;
+  const int rc = fzi::set_kz_chunk(h, h->kz_chunk > 0 ? h->kz_chunk : 0);
+  h->finalized = rc == FZ_OK;
+  return rc;
 }
 
 template <class R>
@@ -1010,20 +1006,32 @@ dim3 plan_grid(const fz_handle* h, size_t chunks) {
   return dim3((unsigned)ntx, (unsigned)nty, (unsigned)(chunks * h->nb));
 }
 
-void set_plan(fz_handle* h, StagePlan p, bool z_auto) {
+int set_plan(fz_handle* h, StagePlan p, bool z_auto) {
+  if (!p.direct) {
+    const int rc = need_band_workspace(h);
+    if (rc != FZ_OK) return rc;
+  }
   const bool same = p.zsizes == h->zsizes && p.grid.x == h->stage_grid.x && p.grid.y == h->stage_grid.y &&
                     p.grid.z == h->stage_grid.z && p.direct == h->direct && z_auto == h->z_auto;
   swap_plan(h, p);
   h->z_auto = z_auto;
-  if (same) return;
+  if (same) return FZ_OK;
   h->launch_gen++;
   for (auto& g : h->graph)
     if (g) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
+  return FZ_OK;
 }
 }  // namespace
+
+int need_band_workspace(fz_handle* h) {
+  if (h->d_wst || h->nB == 0 || h->K > 4 || h->L > 4) return FZ_OK;
+  FZ_CUDA(h, cudaMalloc(&h->d_wst, (size_t)h->nB * 2 * 8), "cudaMalloc(band workspace)");
+  h->launch_gen++;
+  return FZ_OK;
+}
 
 void swap_plan(fz_handle* h, StagePlan& p) {
   std::swap(h->zsizes, p.zsizes);
@@ -1053,13 +1061,12 @@ int set_z_sizes(fz_handle* h, const std::vector<int>& sizes) {
   if (sizes.empty() || (int)sizes.size() > fz::FZ_MAX_ZCHUNKS || sum != nzi)
     return set_error(h, FZ_EINVAL, "z chunks must cover the interior planes in at most " +
                                        std::to_string(fz::FZ_MAX_ZCHUNKS) + " pieces");
-  set_plan(h, StagePlan{sizes, plan_grid(h, sizes.size()), false}, false);
-  return FZ_OK;
+  return set_plan(h, StagePlan{sizes, plan_grid(h, sizes.size()), false}, false);
 }
 
-void set_kz_chunk(fz_handle* h, int kz_chunk) {
+int set_kz_chunk(fz_handle* h, int kz_chunk) {
   const bool z_auto = kz_chunk <= 0;
-  set_plan(h, uniform_plan(h, z_auto ? h->kz_heuristic : kz_chunk, z_auto && h->direct_rule), z_auto);
+  return set_plan(h, uniform_plan(h, z_auto ? h->kz_heuristic : kz_chunk, z_auto && h->direct_rule), z_auto);
 }
 
 StageTiles stage_tiles(const fz_handle* h) {

@@ -471,7 +471,8 @@ int fz_group_create(fz_handle* const* members, int32_t n, fz_group** out) {
       if (members[j] == members[i]) return fzi::set_global_error(FZ_EINVAL, "fz_group_create: repeated member");
   }
   for (int i = 0; i < n; i++) {
-    const int rc = fzi::prepare(members[i]);
+    int rc = fzi::prepare(members[i]);
+    if (rc == FZ_OK) rc = fzi::need_band_workspace(members[i]);
     if (rc != FZ_OK) return fzi::set_global_error(rc, "fz_group_create: member " + std::to_string(i) + ": " + members[i]->err);
   }
   fz_group* g = new (std::nothrow) fz_group();

@@ -66,7 +66,9 @@ struct fz_handle {
   void* d_bnrm = nullptr;
   double* d_ade[3][3] = {{nullptr}};  // [set][phi, psi1, psi2]
   int ph_old = 0, ph_cur = 1, ph_nu = 2;
-  double* d_wst = nullptr;  // outgoing characteristics of stages 0 and 1 of a step, per band record
+  // outgoing characteristics of stages 0 and 1 of a step, per band record: for the separate band kernel of
+  // up to 4 real poles and 4 pairs, allocated when launches with it are first chosen
+  double* d_wst = nullptr;
   bool keep_ade = false;    // the band kernels store the states after every stage (the adjoint's recompute)
 
   // materials
@@ -183,9 +185,11 @@ cudaError_t enqueue_finish(fz_handle* h);
 int bind_field_set(fz_handle* h, int set, void* const* f);
 // the stage kernel of stage st alone (no band), on the handle's stream: the autotuner's trial
 cudaError_t enqueue_stage_kernel(fz_handle* h, int st);
-// tile depth of the stage kernels (z planes per CTA; 0 = the wave-filling heuristic); drops the
-// handle's captured graphs
-void set_kz_chunk(fz_handle* h, int kz_chunk);
+// the workspace of the separate band kernel, if the handle's band takes one and has none yet
+int need_band_workspace(fz_handle* h);
+// tile depth of the stage kernels (z planes per CTA; 0 = the heuristic); drops the handle's captured
+// graphs
+int set_kz_chunk(fz_handle* h, int kz_chunk);
 // z chunks of any lengths (summing to the interior planes, at most FZ_MAX_ZCHUNKS) of the marching
 // stage kernel; drops graphs
 int set_z_sizes(fz_handle* h, const std::vector<int>& sizes);

@@ -449,6 +449,15 @@ __global__ void FZ_BAND_BOUNDS(R, KM) k_band(const __grid_constant__ BandArgs<R>
   band_body<R, STAGE, KM, LM, KEEP>(B, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// The band record of every band cell, for the direct kernel. (Filled on the host and uploaded, an int32 a
+// cell, it took 0.2 of the 1.25 ms that preparing a 256 x 256 plane took, 0.6 of 1.75 for 60 x 50 x 44 cells.)
+__global__ void k_band_index(const int4* __restrict__ rec, int64_t nB, int32_t* __restrict__ index) {
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nB) return;
+  const int4 rc = rec[b];
+  index[((uint64_t)(uint32_t)rc.y << 32) | (uint32_t)rc.x] = (int32_t)b;
+}
+
 // Receiver gather after the last stage of a step (main3D.cu:1399-1414), into a device buffer; then
 // advances the device step counter. One block. off: steps completed since the counter's value (those
 // before the last one were recorded by the stage 0 launches that followed them).
@@ -707,6 +716,13 @@ cudaError_t launch_stage(int stage, bool two_d, const StageArgs<R>& a, const Sta
     else
       k_stage<R, 2, true><<<grid, block, smem, s>>>(a, m);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_band_index(const int4* rec, int64_t nB, int32_t* index, size_t n, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(index, 0xff, n * sizeof(int32_t), s);
+  if (e != cudaSuccess || nB <= 0) return e;
+  k_band_index<<<(unsigned)((nB + 255) / 256), 256, 0, s>>>(rec, nB, index);
   return cudaGetLastError();
 }
 

@@ -25,6 +25,8 @@ DirectShape direct_shape(int Nx, int Ny, int Nz, int nb, bool two_d, int nsm);
 template <class R>
 cudaError_t launch_stage_direct(int stage, bool two_d, const StageArgs<R>& a, const BandArgs<R>& b,
                                 const DirectArgs& d, dim3 grid, cudaStream_t s);
+// index[cell] = band record of the cell, -1 without (n cells)
+cudaError_t launch_band_index(const int4* rec, int64_t nB, int32_t* index, size_t n, cudaStream_t s);
 template <class R>
 cudaError_t launch_band(int stage, const BandArgs<R>& a, cudaStream_t s);
 template <class R>

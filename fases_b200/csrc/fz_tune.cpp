@@ -101,8 +101,7 @@ namespace fzi {
 
 int apply_z_plan(fz_handle* h, const ZPlan& p) {
   if (p.guided) return set_z_sizes(h, guided_z_sizes(h, p.depth));
-  set_kz_chunk(h, p.depth);
-  return FZ_OK;
+  return set_kz_chunk(h, p.depth);
 }
 
 std::vector<ZPlan> kz_candidates(fz_handle* h) {
@@ -254,8 +253,7 @@ int fz_set_kz_chunk(fz_handle* h, int32_t kz_chunk) {
   if (rc != FZ_OK) return rc;
   // the depth that fz_autotune gives where the direct kernel won
   if (h->direct_rule && kz_chunk == h->kz_heuristic) kz_chunk = 0;
-  fzi::set_kz_chunk(h, kz_chunk);
-  return FZ_OK;
+  return fzi::set_kz_chunk(h, kz_chunk);
 }
 
 int fz_get_z_schedule(fz_handle* h, int32_t* sizes, int32_t cap, int32_t* n) {
@@ -278,10 +276,8 @@ int fz_set_z_schedule(fz_handle* h, const int32_t* sizes, int32_t n) {
   rc = fz_sync(h, 0);
   if (rc != FZ_OK) return rc;
   const std::vector<int> z(sizes, sizes + n);
-  if (h->direct_rule && z == fzi::uniform_plan(h, h->kz_heuristic, true).zsizes) {  // as fz_set_kz_chunk
-    fzi::set_kz_chunk(h, 0);
-    return FZ_OK;
-  }
+  if (h->direct_rule && z == fzi::uniform_plan(h, h->kz_heuristic, true).zsizes)  // as fz_set_kz_chunk
+    return fzi::set_kz_chunk(h, 0);
   return fzi::set_z_sizes(h, z);
 }
 
