@@ -143,6 +143,11 @@ constexpr int32_t KERR_BOUNDS = 4;     // the bounds-checked build caught an ind
 // Index check of the bounds-checked build (compiled with -DFZ_BOUNDS_CHECK): an index outside
 // [0, n) sets KERR_BOUNDS in the error word and the access is skipped. In the normal build the
 // check is the constant true and costs nothing.
+#ifdef FZ_BOUNDS_CHECK
+typedef int64_t cell_offset;  // wide enough to see an offset that 32 bits would wrap
+#else
+typedef uint32_t cell_offset;
+#endif
 #if defined(__CUDACC__)
 __device__ __forceinline__ bool fz_inb(int32_t* err, int64_t i, int64_t n) {
 #ifdef FZ_BOUNDS_CHECK

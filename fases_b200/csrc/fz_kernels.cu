@@ -252,15 +252,15 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
   int buf = 0;
   uint32_t parity = 0;
   // 32-bit offsets: 12 field arrays of 2^32 elements do not fit the device
-  const uint32_t plane32 = (uint32_t)plane;
-  uint32_t gk = (uint32_t)(col + plane * kb);          // offset of (i, j, k)
-  uint32_t gz = (uint32_t)(colz + plane * (kb + 4));  // z-queue load of the next iteration (plane k + 4)
+  const cell_offset planeo = (cell_offset)plane;
+  cell_offset gk = (cell_offset)(col + plane * kb);          // offset of (i, j, k)
+  cell_offset gz = (cell_offset)(colz + plane * (kb + 4));  // z-queue load of the next iteration (plane k + 4)
   // two planes an iteration (FP32): the queue's moves between planes and the buffer parity fall away
   // (500 x 400 x 200, with the 32-bit offsets and the common row pitch above: a stage 0.685 / 0.716 /
   // 0.718 ms, one plane an iteration 0.708 / 0.728 / 0.731; three 0.719 / 0.778 / 0.782, four 0.707 /
   // 0.737 / 0.741, both spilling)
 #pragma unroll (sizeof(R) == 4 && !DIM2 ? CTA::planes : 1)
-  for (int it = 0; it < nplanes; ++it, gk += plane32, gz += plane32) {
+  for (int it = 0; it < nplanes; ++it, gk += planeo, gz += planeo) {
     const int k = kb + it;
     X* Xlo = reinterpret_cast<X*>(cbase) + (it & 1) * (2 * L::XC + 2 * L::YC);
     X* Xhi = Xlo + L::XC;
@@ -356,7 +356,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
 
     // ---- the RK update of this cell before its cPML and source terms: differences across the cell
     //      along each axis (.x pressure, .y velocity), stage combination
-    auto rk_update = [&](uint32_t g, P& Dx, P& Dy, P& Dz, R& pn, R& un, R& vn, R& wn) {
+    auto rk_update = [&](cell_offset g, P& Dx, P& Dy, P& Dz, R& pn, R& un, R& vn, R& wn) {
       Dx = Sw::across(A, Xlo[ty * L::CP + tx], xhi, xlo, Xhi[ty * L::CP + tx + 2]);
       Dy = Sw::across(A, Ylo[ty * L::CP + tx], yhi, ylo, Yhi[(ty + 2) * L::CP + tx]);
       Dz = Sw::across(Fz_lo, Fz_hi);
@@ -387,7 +387,7 @@ __device__ __forceinline__ void stage_body(const StageArgs<R>& A, const StageMap
       A.vo[gk] = vn;
       A.wo[gk] = wn;
     } else if (valid && (cls & (CLS_UPDATE | CLS_SOURCE)) && fz_inb(A.err, gk, A.nfield)) {
-      const uint32_t g = gk;
+      const cell_offset g = gk;
       if (cls & CLS_UPDATE) {
         P Dx, Dy, Dz;
         R pn, un, vn, wn;
