@@ -214,8 +214,8 @@ struct BandArgs {
   int64_t nfield;  // elements of one field array (bounds-checked build)
 };
 
-// The direct stage kernel of small rooms (fz_direct.cu): march depth of a warp and chunks of it per
-// member along z, and the band index of every cell (-1: none).
+// The direct stage kernel of small rooms (fz_direct.cu): rows a warp marches over in a planar room, planes
+// of a member (1 in a planar room), and the band index of every cell (-1: none).
 constexpr int DIRECT_CELLS = 30;  // cells of a row a warp of it updates
 
 struct DirectArgs {

@@ -5,10 +5,9 @@
 // many planes to run well; a room of 10^4 to 10^6 cells gives it a handful of CTAs whose planes run
 // one after another (26 x 22 x 18 cells: 4 CTAs x 9 planes, 25 us a stage; 71 x 53 x 47: 60 CTAs x 10
 // planes, 28 us), and the band list one more dependent launch. Here
-//  - a warp owns 30 cells of a row (lanes 0 and 31 are the halo centres) for a few planes: x centres
-//    once per lane, exchanged by shuffles; y centres of the rows below and above recomputed (three a
-//    cell instead of one); z centres from a register queue, as the marching kernel. No shared memory,
-//    no barrier: all loads of a cell are independent and hit L1 / L2;
+//  - a warp owns 30 cells of a row (lanes 0 and 31 are the halo centres): x centres once per lane,
+//    exchanged by shuffles; y and z centres of the rows below and above recomputed (three a cell instead
+//    of one). No shared memory, no barrier: all loads of a cell are independent and hit L1 / L2;
 //  - the thread that updated a band cell runs its ADE boundary at once (the probe reads the stage
 //    input), which saves the band launch.
 // About twice the marching kernel's arithmetic a cell, so it is the better one only while the GPU is
@@ -17,7 +16,8 @@
 // chained loads (stencil, band record, probe: seven of the twelve cycles between two instructions of a
 // warp, by its stall counters) and the launches. Five or six CTAs an SM (96, 80 registers) measured 17
 // and 18 us; programmatic dependent launches 16.7 where plain ones took 16.0.
-// A planar room marches along y (no barrier and no redundant centres there).
+// A planar room marches along y, a warp one row or (FP64 planes near the line) two: no barrier there, and
+// the second row's centres come from the first's registers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -219,16 +219,15 @@ cudaError_t launch(int fit, const StageArgs<R>& a, const BandArgs<R>& b, const D
 DirectShape direct_shape(int Nx, int Ny, int Nz, int nb, bool two_d, int nsm) {
   DirectShape sh;
   const int ex = Nx - 2 * GHOST, ey = Ny - 2 * GHOST, ez = Nz - 2 * GHOST;
-  const int64_t rows = (int64_t)((ex + DCELLS - 1) / DCELLS) * nb * (two_d ? 1 : ey);  // warps per marched cell
-  const int len = two_d ? ey : ez;
-  // a march of one cell pays for two extra centres (of 4 or 6), so it deepens as soon as the warps
-  // keep every scheduler busy without it
-  const int64_t want = (int64_t)nsm * 16;
-  sh.depth = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)len, 8, rows * len / want}));
-  sh.chunks = two_d ? 1 : (len + sh.depth - 1) / sh.depth;
-  const int warps_y = two_d ? (len + sh.depth - 1) / sh.depth : ey;
-  sh.grid = dim3((unsigned)((ex + DCELLS - 1) / DCELLS), (unsigned)((warps_y + DROWS - 1) / DROWS),
-                 (unsigned)(sh.chunks * nb));
+  const int tiles = (ex + DCELLS - 1) / DCELLS;
+  // a planar march of one row pays for two extra centres (of 4), so it takes two rows as soon as the warps
+  // keep every scheduler busy without it. 3D rooms of so many warps run the marching kernel: their marches
+  // are of one plane (compiled without the loop, the 3D form takes 17.2 instead of 16.0 us a step of 26 x 22
+  // x 18 cells, 28.0 instead of 26.5 of 45 x 38 x 29 FP64: 128 registers in every instance, and other spills)
+  sh.depth = two_d && ey > 1 && (int64_t)tiles * nb * ey >= 32 * (int64_t)nsm ? 2 : 1;
+  sh.chunks = two_d ? 1 : ez;
+  const int warps_y = (ey + sh.depth - 1) / sh.depth;
+  sh.grid = dim3((unsigned)tiles, (unsigned)((warps_y + DROWS - 1) / DROWS), (unsigned)(sh.chunks * nb));
   return sh;
 }
 

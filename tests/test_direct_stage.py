@@ -1,6 +1,6 @@
 """The direct stage kernel of small rooms (fz_direct.cu) against the marching kernel: the same
 arithmetic per cell, so traces and fields agree bit for bit. Shapes at the edges of its tiles (30
-cells of a row per warp, 4 rows per CTA, marches of 1 to 8 cells), every pole form of the band,
+cells of a row per warp, 4 rows per CTA, planar marches of one row and of two), every pole form of the band,
 cPML on any face, sources in air and in skipped cells, batches and planar rooms."""
 import numpy as np
 import pytest
@@ -46,7 +46,8 @@ CASES = [
     ((26, 22, 18), {"K": 0, "L": 0}), ((20, 15, 11), {"batch": 3}), ((90, 1, 40), {}), ((4, 70, 60), {}),
     ((64, 61), {"two_d": True}), ((30, 257), {"two_d": True, "pml": (0, 0, 1, 1, 1, 0)}),
     ((250, 90), {"two_d": True, "K": 3, "L": 0}), ((33, 40), {"two_d": True, "batch": 2}),
-    ((700, 250), {"two_d": True}),  # several cells per march
+    ((700, 250), {"two_d": True}),  # FP64: two rows per march
+    ((690, 253), {"two_d": True}),  # FP64: and one row in the last
 ]
 
 
