@@ -52,7 +52,10 @@ __device__ __forceinline__ void record_samples(const R* p, const R* u, const R* 
   }
 }
 // The previous step's samples, by the threads of one block of a stage 0 launch: the step's result is
-// the stage's input, so this needs no launch of its own between the steps.
+// the stage's input, so this needs no launch of its own between the steps. Many receivers lengthen that
+// block, about as much as they did their own launch: us a step with 16 / 4096 / 20000 receivers, by a launch
+// -> here, 26 x 22 x 18 FP32 74 / 94 / 171 -> 15 / 38 / 125, 119 x 103 x 87 130 / 155 / 253 -> 122 / 144 / 251,
+// 250 x 200 x 150 582 / 608 / 713 -> 556 / 559 / 651, where other blocks hide part of it.
 template <class R>
 __device__ __noinline__ void stage_receivers(const StageArgs<R>& A, int t, int nt) {
   record_samples<R>(A.pi, A.ui, A.vi, A.wi, A.rcell, A.rec_n, A.ir, A.vel, A.rec_cap, *A.step + A.rec_off, A.err,
@@ -153,11 +156,12 @@ __device__ __forceinline__ void ade_pair(double& r1, double& r2, double m1, doub
 // KEEP: the pole states after this stage are stored (the left role), and the stage reads its right and
 // middle sets. Otherwise only the last stage stores states: the recursion is linear in the state at
 // step start and the outgoing characteristics, so stages 1 and 2 recompute the earlier stages' states
-// from those (8 bytes a stage, kept in wst) instead of reading and writing sets of 8 (K + 2L) bytes.
-// With K = L = 2 a band cell moves 176 instead of 384 bytes of states a step, with the same bits:
+// from those (8 bytes a stage, kept in wst) instead of reading and writing sets of 8 (K + 2L) bytes: every
+// stage reads the set of step start. With K = L = 2 a band cell moves 232 instead of 384 bytes of states
+// and characteristics a step, with the same bits:
 // 500 x 400 x 200 cells (2.35 M band cells) 120 us a launch instead of 137, 190 x 150 x 140 FP64 39
-// instead of 44. By its counters (192^3) the kernel then reads 231 bytes of DRAM a cell and launch, 58 %
-// of the copy rate: band rows of walls normal to x are three cells long, a third of a sector.
+// instead of 44. By its counters (192^3) the kernel then reads 223 to 239 bytes of DRAM a cell and launch,
+// 59 % of the peak rate: band rows of walls normal to x are three cells long, a third of a sector.
 // KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
 // probe is then issued at the top, beside the probe gathers, so one thread keeps ~50 loads in flight;
 // KM = LM = 0 is the general form with the state loads inside the pole loops; it keeps every state.

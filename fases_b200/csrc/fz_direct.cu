@@ -11,9 +11,9 @@
 //  - the thread that updated a band cell runs its ADE boundary at once (the probe reads the stage
 //    input), which saves the band launch.
 // About twice the marching kernel's arithmetic a cell, so it is the better one only while the GPU is
-// not full; use_direct (fz_api.cpp) draws the line. 26 x 22 x 18 FP32 takes 15 us a step (marching in
+// not full; use_direct (fz_api.cpp) draws the line. 26 x 22 x 18 FP32 takes 15 to 16 us a step (marching in
 // chunks of 9 planes: 72), 45 x 38 x 29 FP64 26 (10 planes: 107). What is left is the latency of the
-// chained loads (stencil, band record, probe: seven of the twelve cycles between two instructions of a
+// chained loads (stencil, band record, probe: five to six of the ten cycles between two instructions of a
 // warp, by its stall counters) and the launches. Five or six CTAs an SM (96, 80 registers) measured 17
 // and 18 us; programmatic dependent launches 16.7 where plain ones took 16.0.
 // A planar room marches along y, a warp one row or (FP64 planes near the line) two: no barrier there, and

@@ -113,7 +113,7 @@ struct fz_handle {
   int32_t* d_err = nullptr;
 
   // step counter and bookkeeping
-  // workspaces of fz_get_fields, kept while they are small (PACK_KEEP bytes)
+  // workspaces of fz_get_fields: 4 MB (or one row, if longer) at most each, kept
   void* d_pack = nullptr;
   size_t pack_bytes = 0;
   std::unique_ptr<char[]> pack_host;  // pack_host_bytes

@@ -116,7 +116,7 @@ struct StageSmem {
 // the stage (main3D.cu:1288, 1296, 1304).
 // ------------------------------------------------------------------------------------------
 #ifndef FZ_STAGE_MINBLOCKS_F32
-#define FZ_STAGE_MINBLOCKS_F32 (1024 / NTHREADS)  // 32 warps per SM in FP32 (64 registers, no spills)
+#define FZ_STAGE_MINBLOCKS_F32 (1024 / NTHREADS)  // 32 warps per SM in FP32 (64 registers, 16 bytes spilled)
 #endif
 // DIM2: planar solve (one updated z-plane, no z fluxes): the 3D scheme restricted to 2D.
 // CTA coordinates of a stage-kernel launch of one room: the launch grid itself.

@@ -8,7 +8,7 @@
 //   - every node's centre is reconstructed once per direction for both its faces, by one thread, and
 //     its two outgoing characteristics p -+ rho c u go to shared memory (34 x 6 nodes for x, 32 x 8
 //     for y: one pass of the 256 threads each), where the reference reconstructs every face twice, once
-//     from each side. 803 x 815 nodes FP32: 52 us a step; with the reference's six IEEE divisions and
+//     from each side. 803 x 815 nodes FP32: 53 us a step; with the reference's six IEEE divisions and
 //     double-precision indicators per face value it was 198. A 32 x 14 tile with 512 threads takes 54;
 //   - fluid nodes (S >= h) get the stage update and the multiplicative sPML;
 //   - the nodes of rows 3, Ny-5 and Ny-4 write the ghost rows of p and v of their column;
@@ -83,10 +83,11 @@ struct Args {
 // the Godunov flux, as fz_pair.cuh evaluates them for the FP64 3D scheme. The indicators are quadratic forms
 // of first differences, which are exact where the field is smooth; the reference forms second
 // differences from the values themselves (rounding at the size of p) and squares those in double.
-// FP32, 803 x 815 nodes, 400 steps, ten seeds: the error against 64 bits is 1.00, 0.98 and 0.66 of that
-// form's for p, u and v, 0.82 for the traces (geometric means). Exchanging only the reconstructed parts and
-// differencing the nodes' own exactly gave 0.93, 0.92, 0.65 and 0.79, inside the seeds' spread, for 1.6 %
-// of the time.
+// FP32, 40 grids of 90 to 900 nodes an edge, 100 to 400 steps: the error against 64 bits is 0.93, 0.91, 0.74 and
+// 0.78 of that form's for p, u, v and the trace (geometric means) at the reference's start of 0.1 Pa, 0.61 to
+// 0.76 at 1e-3 of it, 0.69 to 0.79 at 100 and 0.69 to 0.73 at 1000 times it. Indicators in double, or only the
+// reconstructed parts exchanged, are inside the same spread (0.92 to 0.97 and 0.67 to 0.91) for 9 and 2 % of
+// the time.
 template <class R>
 __device__ __forceinline__ void js_waves(const R* fp, const R* fv, int st, R eps, R Z0, R& wr, R& wl) {
   fz::weno_waves<R, fz::WENO_BOTH, fz::WenoJS>(fz::pmk(fp[-2 * st], fv[-2 * st]), fz::pmk(fp[-st], fv[-st]),
