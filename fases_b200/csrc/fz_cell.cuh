@@ -160,8 +160,8 @@ __device__ __forceinline__ void ade_pair(double& r1, double& r2, double m1, doub
 // stage reads the set of step start. With K = L = 2 a band cell moves 232 instead of 384 bytes of states
 // and characteristics a step, with the same bits:
 // 500 x 400 x 200 cells (2.35 M band cells) 120 us a launch instead of 137, 190 x 150 x 140 FP64 39
-// instead of 44. By its counters (192^3) the kernel then reads 223 to 239 bytes of DRAM a cell and launch,
-// 59 % of the peak rate: band rows of walls normal to x are three cells long, a third of a sector.
+// instead of 44. By its counters (192^3) the kernel then reads 230 to 246 bytes of DRAM a cell and launch,
+// 55 to 59 % of the peak rate: band rows of walls normal to x are three cells long, a third of a sector.
 // KM, LM > 0: at most KM real poles and LM complex pairs. Every load that does not depend on the
 // probe is then issued at the top, beside the probe gathers, so one thread keeps ~50 loads in flight;
 // KM = LM = 0 is the general form with the state loads inside the pole loops; it keeps every state.

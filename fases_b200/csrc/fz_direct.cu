@@ -33,7 +33,6 @@ namespace {
 
 constexpr int DROWS = 4;  // warps (rows, or row chunks of a planar room) per CTA
 constexpr int DCELLS = DIRECT_CELLS;  // cells of a row a warp updates
-constexpr unsigned FULL = 0xffffffffu;
 
 template <class R, int STAGE, bool DIM2, int KM, int LM>
 __device__ __forceinline__ void direct_body(const StageArgs<R>& A, const BandArgs<R>& B, const DirectArgs& D, int bx,

@@ -114,9 +114,9 @@ __device__ __forceinline__ void weno_center(float2 qm2, float2 qm1, float2 q0, f
 // (it cancels between the sums and their normalisers).
 //
 // Products of indicators leave the range of the type long before the indicators do (B lies between eps
-// and the square of the largest difference), so each form scales by a power of two, which is exact and
-// leaves the bits of every other case alone: a 2D solve with eps = 1e-40, or fields of 1e30, are as good
-// as any.
+// and the square of the largest difference), so each form scales by a power of two, which is exact (but
+// for what falls below the smallest normal number): a 2D solve with eps = 1e-40, or fields of 1e30, are as
+// good as any.
 
 // 2^-e for x = m 2^e, m in [1, 2), given x's upper word (FP64) or bits (FP32); x subnormal or zero: the
 // largest power of two (FP32: x finite)
