@@ -348,7 +348,8 @@ int fz_info(fz_handle* h, int32_t* dims, int64_t* n_band, int64_t* n_update);
 
 /* Per-kernel-kind device time. When enabled, every launch in fz_run is bracketed by CUDA events
  * on the handle's stream; fz_profile_read returns accumulated milliseconds and launch counts for
- * kinds 0..2 = stage kernels 0,1,2; 3 = band kernels; 4 = receiver gather. */
+ * kinds 0..2 = stage kernels 0,1,2; 3 = band kernels (none where a small room's stage kernels include the
+ * band: its time is in kinds 0..2); 4 = receiver gather. Trial launches of the autotuner are not counted. */
 int fz_profile_enable(fz_handle* h, int32_t on);
 int fz_profile_read(fz_handle* h, double* ms, int64_t* launches, int32_t nkinds);
 
