@@ -45,7 +45,8 @@ typedef struct {
   double h;          /* grid spacing [m] (config line 1) */
   double dt;         /* time step [s]: C_CFL h / c in the reference (main.cu:392) */
   double rho, c;     /* air density, speed of sound (main.cu:384-386; T in kelvin) */
-  double eps;        /* WENO-JS epsilon, 1e-7 */
+  double eps;        /* WENO-JS epsilon, 1e-7; any positive value whose square the precision holds (from 6e-20 in
+                        FP32, 1e-150 in FP64) */
   double tol;        /* band width: 3 h (main.cu:82) */
   int pml_n, pml_s, pml_e, pml_w; /* sPML faces y-high, y-low, x-high, x-low (config lines 7-10) */
   int precision;     /* FZ_FP32 (every array FP32, as the reference) or FZ_FP64 */
